@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "la_build.h"
 #include "lc_layout.h"
 #include "rbs_internal.h"
 
@@ -120,7 +121,10 @@ int pick_group(double avg) {
 // Kernel choice.  REFERENCE maps each reference method to this library's
 // kernel of the same kind; AUTO uses a latency/bandwidth cost model of the
 // B200 (constants measured on a B200 with bench.py).
-void select_kernel(ExecBlock &b, const rbs_options &opt, const std::vector<int> &lvl_sizes) {
+// nseg: independent systems of a batch (1 otherwise).  The single-CTA level
+// kernels run them side by side, one per CTA, so their time is the longest
+// system's levels or an even share of the bytes.
+void select_kernel(ExecBlock &b, const rbs_options &opt, const std::vector<int> &lvl_sizes, int nseg) {
     if (!b.tri) {
         if (b.nnz == 0) {
             b.kernel = RBS_K_EMPTY;
@@ -153,11 +157,14 @@ void select_kernel(ExecBlock &b, const rbs_options &opt, const std::vector<int> 
     }
     // AUTO cost model (microseconds).
     double bytes = (double)off * 12.0 + (double)b.m * 24.0;
+    const double ctas = std::max(1, std::min(nseg, 148));
     double passes = 0;
-    for (int w : lvl_sizes) passes += std::max(1.0, std::ceil((double)w * b.group / 1024.0));
-    double t_level = passes * 0.12 + bytes / 180e3 + 4.0;
+    for (int w : lvl_sizes) passes += std::max(1.0, std::ceil((double)w * b.group / (1024.0 * ctas)));
+    double t_level = passes * 0.12 + bytes / (180e3 * ctas) + 4.0;
     double t_sync = (double)b.nlv * 0.9 + bytes / 4.0e6 + 4.0;
-    double t_seq = (double)b.m * 0.012 + bytes / 120e3 + 4.0;
+    // one warp, one row after another: 0.69 us a row measured (8,000 rows with
+    // 1,298 levels: 5.6 ms, against 0.3 us a level in the level kernels)
+    double t_seq = (double)b.m * 0.69 + bytes / 120e3 + 4.0;
     double t_scan = b.bandwidth <= 8 ? bytes * 3.0 / 3.0e6 + 25.0 : 1e30;
     double best = t_sync;
     b.kernel = RBS_K_SYNCFREE;
@@ -619,6 +626,39 @@ static void build_lc(Plan &P, const rbs_options &opt, const std::vector<int> &le
     P.lc_segs.swap(all.segs);
 }
 
+// The cost model chose a single-CTA level kernel for every triangle that has
+// off-diagonal entries, and at least one of them has rows or levels beyond
+// the staged level-ELL kernel's.
+bool wants_la(const Plan &P) {
+    if (P.opt.select != RBS_SELECT_AUTO) return false;
+    bool any = false;
+    for (const ExecBlock &B : P.blocks) {
+        if (!B.tri || B.nnz == B.m) continue;
+        if (B.kernel != RBS_K_LEVEL) return false;
+        any = any || !B.ca_ok;
+    }
+    return any;
+}
+
+void ensure_lc(Plan &P) {
+    if (!P.lc_deferred) return;
+    P.lc_deferred = false;
+    // local levels from the triangles' entries: a recurrence in row order
+    std::vector<int> level((size_t)P.n, 0);
+    parallel_for(P.blocks.size(), [&](size_t b) {
+        const ExecBlock &B = P.blocks[b];
+        if (!B.tri) return;
+        const int *rp = P.rp_pool.data() + B.rp_off;
+        int *lv = level.data() + B.r0;
+        for (int r = 0; r < B.m; ++r) {
+            int top = -1;
+            for (int k = rp[r]; k < rp[r + 1]; ++k) top = std::max(top, lv[P.col_pool[(size_t)k]]);
+            lv[r] = top + 1;
+        }
+    });
+    build_lc(P, P.opt, level);
+}
+
 int host_bfs_levels(const int *cp, const int *ri, int m, std::vector<int> &levelPtr, std::vector<int> &item) {
     return bfs_levels(cp, ri, m, levelPtr, item);
 }
@@ -956,7 +996,7 @@ int analyse_after_levels(Plan &P, int n, int nnz, int substitution, int lv, cons
                 else B.ref_method = 3;
             }
         }
-        select_kernel(B, opt, lvl_sizes[b]);
+        select_kernel(B, opt, lvl_sizes[b], std::max(1, (int)P.seg_rows.size()));
         // The sync-free kernel's lane group.  A deep triangle (32 levels or
         // more) is bound by its level chain, where each level waits for its
         // longest rows: there the group is sized for the rows' tail, the
@@ -1244,7 +1284,24 @@ int analyse_after_levels(Plan &P, int n, int nnz, int substitution, int lv, cons
     }
     // 11. level-chunk records (level_lc.cuh) and the level kernel of every
     //     level triangle
-    build_lc(P, opt, level);
+    // (a plan that runs on the look-ahead kernel leaves them out until they
+    // are exported or saved: every chunk that kernel takes fits these records)
+    P.la.reset();
+    P.lc_deferred = false;
+    if (!opt.host_only && wants_la(P)) {
+        P.la = std::make_shared<LaHost>();
+        if (!la_build(P, *P.la)) P.la.reset();
+    }
+    if (P.la) {
+        P.lc_deferred = true;
+        P.lc_rec64.clear();
+        P.lc_rec32.clear();
+        P.lc_tab.clear();
+        P.lc_segs.clear();
+        for (ExecBlock &B : P.blocks) B.lc_ok = wants_level(B, opt) && B.nnz > B.m;
+    } else {
+        build_lc(P, opt, level);
+    }
     // 12. ELL chunks of single-CTA triangles (the CTA sync-free kernel,
     //    cta_syncfree.cuh): chunks of <= 512 rows and <= 2048 ELL slots,
     //    column-major inside a chunk, padding column -1; built after the
@@ -1631,6 +1688,23 @@ int export_reference(const Plan &P, const std::string &name, std::vector<int> &i
             }
         return RBS_OK;
     }
+    if (name.rfind("la_", 0) == 0) {  // the look-ahead layout (la_layout.h), built on request; empty where it does not apply
+        LaHost H;
+        la_build(P, H);
+        if (!H.ok) return put(std::vector<int>{});
+        if (name == "la_dim")
+            return put(std::vector<int>{H.dim.xw, H.dim.nm, H.dim.nh, H.dim.q, H.dim.nx, H.dim.slots(8), H.dim.slots(4),
+                                        H.dim.rec_bytes(8), LA_AUX, LA_AHEAD});
+        if (name == "la_tab") {
+            std::vector<int> t(H.tab.size() * LA_TAB_INTS);
+            if (!t.empty()) std::memcpy(t.data(), H.tab.data(), t.size() * sizeof(int));
+            return put(t);
+        }
+        if (name == "la_segs") return put(H.segs);
+        if (name == "la_rec") return put(std::vector<int>(H.rec.begin(), H.rec.end()));
+        if (name == "la_old") return put(std::vector<int>(H.old.begin(), H.old.end()));
+    }
+    if (name.rfind("lc_", 0) == 0) ensure_lc(const_cast<Plan &>(P));
     if (name == "lc_tab") return put(P.lc_tab);
     if (name == "lc_segs") return put(P.lc_segs);
     if (name == "lc_rec64" || name == "lc_rec32") {  // 16-byte-aligned words, returned as int32

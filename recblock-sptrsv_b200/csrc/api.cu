@@ -468,6 +468,11 @@ int rbs_ic0_device(const int *d_rowptr, const int *d_colidx, const double *d_val
 int rbs_plan_save(const rbs_plan *plan, const char *path) {
     if (!plan || !path) return fail(RBS_ERR_ARG, "rbs_plan_save: NULL argument");
     std::string err;
+    try {
+        rbs::ensure_lc(const_cast<rbs::Plan &>(plan->p));
+    } catch (const std::bad_alloc &) {
+        return fail(RBS_ERR_NOMEM, "rbs_plan_save: out of host memory");
+    }
     int rc = rbs::plan_save(plan->p, path, err);
     if (rc) return fail(rc, err);
     return RBS_OK;

@@ -33,6 +33,7 @@
 #include <utility>
 #include <vector>
 
+#include "la_layout.h"
 #include "rbs.h"
 
 namespace rbs {
@@ -200,6 +201,18 @@ struct RefPack {
     std::vector<int> lvl_ptr, lvl_item, m_lv, off_lv, nnz_lv;
 };
 
+// Look-ahead level layout of the whole matrix (la_layout.h): one LaChunk (4
+// ints) per chunk, 2 ints per segment (first chunk, chunks; most work first).
+// Derived from the processing-order CSR when a plan's device state is built;
+// not part of a saved plan.
+struct LaHost {
+    bool ok = false;
+    LaDim dim{};
+    bulk_vector<LaChunk> tab;
+    std::vector<int> segs;
+    bulk_vector<uint32_t> rec;  // FP64 records (the FP32 ones are made from them on the device)
+    bulk_vector<int> old;       // positions of the old entries
+};
 struct Plan {
     int n = 0, nnz = 0, lv = 0, sub = 0, nlevel = 0, sum_block = 0, step = 0;
     rbs_options opt{};
@@ -234,6 +247,11 @@ struct Plan {
     // chunk, chunks, ring offset of the first chunk)
     bulk_vector<uint32_t> lc_rec64, lc_rec32;
     std::vector<int> lc_tab, lc_segs;
+    // Plans that run on the look-ahead kernel leave the level-chunk records
+    // out until they are asked for (ensure_lc); the look-ahead layout is kept
+    // here from the analysis to the upload.
+    bool lc_deferred = false;
+    std::shared_ptr<LaHost> la;
     // original-row offsets of independent systems (batched plans); empty
     // for a single system
     std::vector<int> seg_rows;
@@ -299,6 +317,13 @@ int host_bfs_levels(const int *cp, const int *ri, int m, std::vector<int> &level
 // device_analyse filled
 int analyse_after_levels(Plan &P, int n, int nnz, int substitution, int lv, const rbs_options &opt, std::string &err,
                          const std::vector<int> *seg_rows = nullptr, DevRows *dev_rows = nullptr);
+
+// analysis.cpp: whether the plan's whole walk is the look-ahead kernel's work
+bool wants_la(const Plan &P);
+// analysis.cpp: builds the level-chunk records a plan left out
+void ensure_lc(Plan &P);
+// la_build.h; false: the structure does not suit the kernel
+bool la_build(const Plan &P, LaHost &H);
 
 // ilu0.cu: ILU(0) of a device CSR matrix into d_lu (A's pattern)
 int device_ilu0(const int *d_rp, const int *d_ci, const double *d_val, int n, int nnz, double *d_lu,

@@ -18,6 +18,7 @@
 #include "cta_syncfree.cuh"
 #include "level_ca.cuh"
 #include "level_lc.cuh"
+#include "level_la.cuh"
 #include "rbs_internal.h"
 
 namespace rbs {
@@ -68,6 +69,16 @@ struct DeviceState {
     LcChunk *lc_tab = nullptr;
     LcSeg *lc_segs = nullptr;
     int *lc_queue = nullptr;                              // one segment counter per triangle
+    // look-ahead level layout of the whole matrix (level_la.cuh); with it
+    // every walk is one launch and the blocks' own pools are not uploaded
+    bool la = false;
+    LaDim la_dim{};
+    LaChunk *la_tab = nullptr;
+    int2 *la_segs = nullptr;
+    uint32_t *la_rec64 = nullptr, *la_rec32 = nullptr;
+    int *la_old = nullptr;
+    int la_nseg = 0, la_gather = 0;
+    int *la_queue = nullptr;  // one segment counter per column
     cudaStream_t side = nullptr;                         // L2 prefetch stream; moves of the overlapped walk
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     double **iotab = nullptr;                            // caller's columns for the overlapped walk (k_set_io)
@@ -261,6 +272,7 @@ template <> struct Pools<double> {
     static const double *ellv(const DeviceState &D) { return D.ell_val; }
     static const double *cav(const DeviceState &D) { return D.ca_val; }
     static const unsigned char *lcrec(const DeviceState &D) { return reinterpret_cast<const unsigned char *>(D.lc_rec64); }
+    static const uint32_t *larec(const DeviceState &D) { return D.la_rec64; }
     static double *bw(const DeviceState &D) { return D.bw64; }
     static double *xw(const DeviceState &D) { return D.xw64; }
     static bool &dirty(DeviceState &D) { return D.xw_dirty64; }
@@ -274,6 +286,7 @@ template <> struct Pools<float> {
     static const float *ellv(const DeviceState &D) { return D.ell_val32; }
     static const float *cav(const DeviceState &D) { return D.ca_val32; }
     static const unsigned char *lcrec(const DeviceState &D) { return reinterpret_cast<const unsigned char *>(D.lc_rec32); }
+    static const uint32_t *larec(const DeviceState &D) { return D.la_rec32; }
     static float *bw(const DeviceState &D) { return D.bw32; }
     static float *xw(const DeviceState &D) { return D.xw32; }
     static bool &dirty(DeviceState &D) { return D.xw_dirty32; }
@@ -409,6 +422,7 @@ template <typename VT> int ca_group(const ExecBlock &B, int K) {
 // then the plan's columns per CTA.
 template <typename VT> int plan_group(const Plan &P, int K) {
     if (K == 1) return 0;
+    if (P.dev->la) return 1;  // the look-ahead kernel: one CTA per column, columns contiguous
     int G = 2;
     for (const ExecBlock &B : P.blocks) {
         if (!B.tri || B.nnz == B.m) continue;
@@ -756,11 +770,61 @@ int move_reserve(const DeviceState &D, size_t ca_min) {
     return (int)need;
 }
 
+// Whole-matrix walk of the look-ahead kernel: one launch, K columns side by side.
+template <typename VT, int Q>
+int launch_la_q(DeviceState &D, const LaArgs<VT> &a, int K, std::string &err) {
+    static std::atomic<unsigned long long> attr{0};
+    if (!attr_done(attr)) {
+        CK(cudaFuncSetAttribute(k_tri_la<VT, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, LA_SMEM));
+        attr_mark(attr);
+    }
+    const int smem = a.d.fixed_bytes(sizeof(VT)) + a.slots * a.d.slot_bytes(sizeof(VT));
+    const dim3 grid((unsigned)std::max(1, std::min(a.nseg, D.num_sms)), (unsigned)K);
+    k_tri_la<VT, Q><<<grid, a.d.nm + a.d.nh + 32 * (a.gather + 1), smem, D.stream>>>(a);
+    CK(cudaGetLastError());
+    return RBS_OK;
+}
+
+template <typename VT>
+int launch_la(Plan &P, int K, std::string &err) {
+    DeviceState &D = *P.dev;
+    LaArgs<VT> a{};
+    a.tab = D.la_tab;
+    a.segs = D.la_segs;
+    a.nseg = D.la_nseg;
+    a.rec = reinterpret_cast<const unsigned char *>(Pools<VT>::larec(D));
+    a.old = D.la_old;
+    a.b = Pools<VT>::bw(D);
+    a.x = Pools<VT>::xw(D);
+    a.n = P.n;
+    a.queue = D.la_queue;
+    a.status = D.status;
+    a.limit = P.opt.spin_limit;
+    a.d = D.la_dim;
+    a.slots = a.d.slots(sizeof(VT));
+    a.gather = D.la_gather;
+    CK(cudaMemsetAsync(D.la_queue, 0, sizeof(int) * (size_t)K, D.stream));
+    return a.d.q == 4   ? launch_la_q<VT, 4>(D, a, K, err)
+           : a.d.q == 8 ? launch_la_q<VT, 8>(D, a, K, err)
+                        : launch_la_q<VT, 12>(D, a, K, err);
+}
+
 // One pass over all blocks: triangles solve into xw, squares update bw.
 template <typename VT, int K>
 int launch_blocks(Plan &P, std::string &err, bool io = false) {
     DeviceState &D = *P.dev;
     cudaStream_t st = D.stream;
+    if (D.la) {  // profiled walks report the whole launch as the first block's time
+        for (const ExecBlock &B : P.blocks) {
+            if (D.profile) CK(cudaEventRecord(D.bev[2 * B.index], st));
+            if (B.index == 0) {
+                const int rc = launch_la<VT>(P, K, err);
+                if (rc) return rc;
+            }
+            if (D.profile) CK(cudaEventRecord(D.bev[2 * B.index + 1], st));
+        }
+        return RBS_OK;
+    }
     const VT *val = Pools<VT>::val(D);
     const VT *inv = Pools<VT>::inv(D);
     VT *bw = Pools<VT>::bw(D);
@@ -1008,6 +1072,7 @@ int launch_blocks(Plan &P, std::string &err, bool io = false) {
 // vector for its sentinel (the sync-free kernels), with the kernel choice
 // of launch_blocks.
 bool walk_polls(const Plan &P, int K) {
+    if (P.dev->la) return false;
     for (const ExecBlock &B : P.blocks) {
         if (!B.tri) continue;
         if (B.kernel == RBS_K_SYNCFREE) return true;
@@ -1028,7 +1093,7 @@ int run_blocks(Plan &P, std::string &err, bool io = false) {
     }
     // per-block timing needs real event timestamps, which captured event
     // records are not: profiled solves launch eagerly
-    if (!D.use_graphs || D.profile) return launch_blocks<VT, K>(P, err, io);
+    if (!D.use_graphs || D.profile || D.la) return launch_blocks<VT, K>(P, err, io);
     const long long key = (long long)K * 8 + (sizeof(VT) == 8 ? 0 : 2) + (io ? 4 : 0);
     auto it = D.graphs.find(key);
     if (it != D.graphs.end()) {
@@ -1125,7 +1190,7 @@ template <int K>
 int solve_fp64(Plan &P, const double *b, double *x, int k, int ld, std::string &err) {
     DeviceState &D = *P.dev;
     const int GL = plan_group<double>(P, K);
-    if (K > 1 && GL) {
+    if (K > 1 && GL && !D.la) {
         int rc = ensure_io_rows(P, err);
         if (rc) return rc;
         k_set_io<<<1, RBS_IO_COLS, 0, D.stream>>>(D.iotab, b, x, ld, k);
@@ -1146,7 +1211,7 @@ template <int K>
 int solve_fp32(Plan &P, const double *b, double *x, int k, int ld, std::string &err) {
     DeviceState &D = *P.dev;
     const int GL = plan_group<float>(P, K);
-    if (K > 1 && GL) {
+    if (K > 1 && GL && !D.la) {
         int rc = ensure_io_rows(P, err);
         if (rc) return rc;
         k_set_io<<<1, RBS_IO_COLS, 0, D.stream>>>(D.iotab, b, x, ld, k);
@@ -1396,28 +1461,45 @@ int solve_k(Plan &P, const double *b, double *x, int k, int ld, int prec, int &i
 
 }  // namespace
 
-int device_build(Plan &P, std::string &err) {
-    if (P.dev) device_free(P);
-    P.dev = new DeviceState();
+namespace {
+
+// Builds and uploads the look-ahead layout (D.la stays false where the
+// structure does not suit it).
+int upload_la(Plan &P, std::string &err) {
     DeviceState &D = *P.dev;
-    if (P.opt.device >= 0) CK(cudaSetDevice(P.opt.device));
-    CK(cudaGetDevice(&D.device));
-    CK(cudaDeviceGetAttribute(&D.num_sms, cudaDevAttrMultiProcessorCount, D.device));
-    CK(cudaDeviceGetAttribute(&D.smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, D.device));
-    CK(cudaDeviceGetAttribute(&D.smem_reserved, cudaDevAttrReservedSharedMemoryPerBlock, D.device));
-    // The walk's stream at the greatest priority, its side stream (prefetch,
-    // the overlapped walk's moves) at the lowest: when both have CTAs
-    // waiting, an SM that frees up takes the walk's.
-    int prio_low = 0, prio_high = 0;
-    CK(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
-    CK(cudaStreamCreateWithPriority(&D.stream, cudaStreamNonBlocking, prio_high));
-    D.own_stream = true;
-    CK(cudaEventCreate(&D.ev0));
-    CK(cudaEventCreate(&D.ev1));
-    {
-        const char *ng = std::getenv("RBS_NO_GRAPHS");
-        D.use_graphs = !(ng && ng[0] == '1');
+    if (!P.la) {
+        P.la = std::make_shared<LaHost>();
+        la_build(P, *P.la);
     }
+    if (!P.la->ok) return RBS_OK;
+    LaHost &H = *P.la;
+    int rc;
+    if ((rc = upload(D, D.la_tab, H.tab, err)) || (rc = upload(D, D.la_rec64, H.rec, err)) ||
+        (rc = upload(D, D.la_old, H.old, err)))
+        return rc;
+    D.la_gather = H.old.empty() ? 0 : 1;
+    std::vector<int2> segs(H.segs.size() / 2);
+    for (size_t q = 0; q < segs.size(); ++q) segs[q] = make_int2(H.segs[2 * q], H.segs[2 * q + 1]);
+    if ((rc = upload(D, D.la_segs, segs, err))) return rc;
+    D.la_nseg = (int)segs.size();
+    if ((rc = alloc(D, D.la_queue, 128, err))) return rc;
+    if (D.mixed) {
+        const size_t nch = H.tab.size();
+        if ((rc = alloc(D, D.la_rec32, nch * H.dim.rec_bytes(4) / 4, err))) return rc;
+        k_la_rec32<<<(unsigned)nch, 128, 0, D.stream>>>(H.dim, reinterpret_cast<const unsigned char *>(D.la_rec64),
+                                                        reinterpret_cast<unsigned char *>(D.la_rec32));
+        CK(cudaGetLastError());
+    }
+    D.la_dim = H.dim;
+    P.la.reset();
+    D.la = true;
+    return RBS_OK;
+}
+
+// The blocks' pools and per-kernel layouts (the block walk).
+int upload_blocks(Plan &P, std::string &err) {
+    DeviceState &D = *P.dev;
+    ensure_lc(P);
     int rc;
     if ((rc = upload(D, D.rp, P.rp_pool, err))) return rc;
     if ((rc = upload(D, D.col, P.col_pool, err))) return rc;
@@ -1425,21 +1507,9 @@ int device_build(Plan &P, std::string &err) {
     if ((rc = upload(D, D.lvl, P.lvl_pool, err))) return rc;
     if ((rc = upload(D, D.map, P.map_pool, err))) return rc;
     if ((rc = upload(D, D.rows, P.rows_pool, err))) return rc;
-    if ((rc = upload(D, D.perm, P.perm, err))) return rc;
-    {
-        std::vector<int> ipos(P.perm.size());
-        for (size_t p = 0; p < P.perm.size(); ++p) ipos[(size_t)P.perm[p]] = (int)p;
-        if ((rc = upload(D, D.ipos, ipos, err))) return rc;
-    }
-    if ((rc = upload(D, D.inv, P.inv_diag, err))) return rc;
-    D.mixed = P.opt.mixed != 0;
     if (D.mixed) {
-        const auto v32 = to_f32(P.val_pool), i32 = to_f32(P.inv_diag);
+        const auto v32 = to_f32(P.val_pool);
         if ((rc = upload(D, D.val32, v32, err))) return rc;
-        if ((rc = upload(D, D.inv32, i32, err))) return rc;
-        if ((rc = upload(D, D.full_rp, P.full_rp, err))) return rc;
-        if ((rc = upload(D, D.full_col, P.full_col, err))) return rc;
-        if ((rc = upload(D, D.full_val, P.full_val, err))) return rc;
     }
     if ((rc = upload(D, D.band_coef, P.band_coef, err))) return rc;
     if ((rc = upload(D, D.band_inv, P.band_inv, err))) return rc;
@@ -1498,6 +1568,53 @@ int device_build(Plan &P, std::string &err) {
         if ((rc = upload(D, D.lc_segs, segs, err))) return rc;
         if ((rc = alloc(D, D.lc_queue, (size_t)(1 << P.lv), err))) return rc;
     }
+    return RBS_OK;
+}
+
+}  // namespace
+
+int device_build(Plan &P, std::string &err) {
+    if (P.dev) device_free(P);
+    P.dev = new DeviceState();
+    DeviceState &D = *P.dev;
+    if (P.opt.device >= 0) CK(cudaSetDevice(P.opt.device));
+    CK(cudaGetDevice(&D.device));
+    CK(cudaDeviceGetAttribute(&D.num_sms, cudaDevAttrMultiProcessorCount, D.device));
+    CK(cudaDeviceGetAttribute(&D.smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, D.device));
+    CK(cudaDeviceGetAttribute(&D.smem_reserved, cudaDevAttrReservedSharedMemoryPerBlock, D.device));
+    // The walk's stream at the greatest priority, its side stream (prefetch,
+    // the overlapped walk's moves) at the lowest: when both have CTAs
+    // waiting, an SM that frees up takes the walk's.
+    int prio_low = 0, prio_high = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
+    CK(cudaStreamCreateWithPriority(&D.stream, cudaStreamNonBlocking, prio_high));
+    D.own_stream = true;
+    CK(cudaEventCreate(&D.ev0));
+    CK(cudaEventCreate(&D.ev1));
+    {
+        const char *ng = std::getenv("RBS_NO_GRAPHS");
+        D.use_graphs = !(ng && ng[0] == '1');
+    }
+    int rc;
+    if ((rc = upload(D, D.perm, P.perm, err))) return rc;
+    {
+        std::vector<int> ipos(P.perm.size());
+        for (size_t p = 0; p < P.perm.size(); ++p) ipos[(size_t)P.perm[p]] = (int)p;
+        if ((rc = upload(D, D.ipos, ipos, err))) return rc;
+    }
+    if ((rc = upload(D, D.inv, P.inv_diag, err))) return rc;
+    D.mixed = P.opt.mixed != 0;
+    if (D.mixed) {
+        const auto i32 = to_f32(P.inv_diag);
+        if ((rc = upload(D, D.inv32, i32, err))) return rc;
+        if ((rc = upload(D, D.full_rp, P.full_rp, err))) return rc;
+        if ((rc = upload(D, D.full_col, P.full_col, err))) return rc;
+        if ((rc = upload(D, D.full_val, P.full_val, err))) return rc;
+    }
+    if (wants_la(P)) {
+        if ((rc = upload_la(P, err))) return rc;
+    }
+    if (!D.la && (rc = upload_blocks(P, err))) return rc;
     {
         int prio_low = 0, prio_high = 0;
         CK(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
@@ -1759,6 +1876,12 @@ void device_free(Plan &P) {
     cudaFree(D.lc_tab);
     cudaFree(D.lc_segs);
     cudaFree(D.lc_queue);
+    cudaFree(D.la_tab);
+    cudaFree(D.la_segs);
+    cudaFree(D.la_rec64);
+    cudaFree(D.la_rec32);
+    cudaFree(D.la_old);
+    cudaFree(D.la_queue);
     cudaFree(D.stage_b);
     cudaFree(D.stage_x);
     void *ptrs[] = {D.rp, D.col, D.lvl, D.map, D.rows, D.perm, D.ipos, D.val, D.inv, D.val32, D.inv32,
