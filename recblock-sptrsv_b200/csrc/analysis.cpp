@@ -19,6 +19,7 @@
 #include "la_build.h"
 #include "lc_layout.h"
 #include "rbs_internal.h"
+#include "strip_build.h"
 
 namespace rbs {
 
@@ -636,6 +637,20 @@ bool wants_la(const Plan &P) {
         if (!B.tri || B.nnz == B.m) continue;
         if (B.kernel != RBS_K_LEVEL) return false;
         any = any || !B.ca_ok;
+    }
+    return any;
+}
+
+// The cost model chose a level kernel for every triangle that has
+// off-diagonal entries, and each of them has the narrow levels and short rows
+// of the staged level-ELL kernel.
+bool wants_strips(const Plan &P) {
+    if (P.opt.select != RBS_SELECT_AUTO || !P.seg_rows.empty()) return false;
+    bool any = false;
+    for (const ExecBlock &B : P.blocks) {
+        if (!B.tri || B.nnz == B.m) continue;
+        if (B.kernel != RBS_K_LEVEL || !B.ca_ok) return false;
+        any = true;
     }
     return any;
 }
@@ -1284,15 +1299,19 @@ int analyse_after_levels(Plan &P, int n, int nnz, int substitution, int lv, cons
     }
     // 11. level-chunk records (level_lc.cuh) and the level kernel of every
     //     level triangle
-    // (a plan that runs on the look-ahead kernel leaves them out until they
-    // are exported or saved: every chunk that kernel takes fits these records)
+    // (a plan that runs on a whole-matrix kernel leaves them out until they
+    // are exported or saved: the rows those kernels take fit these records)
     P.la.reset();
+    P.strip.reset();
     P.lc_deferred = false;
-    if (!opt.host_only && wants_la(P)) {
+    if (!opt.host_only && wants_strips(P)) {
+        P.strip = std::make_shared<StripHost>();
+        if (!strip_build(P, *P.strip)) P.strip.reset();
+    } else if (!opt.host_only && wants_la(P)) {
         P.la = std::make_shared<LaHost>();
         if (!la_build(P, *P.la)) P.la.reset();
     }
-    if (P.la) {
+    if (P.la || P.strip) {
         P.lc_deferred = true;
         P.lc_rec64.clear();
         P.lc_rec32.clear();
@@ -1703,6 +1722,16 @@ int export_reference(const Plan &P, const std::string &name, std::vector<int> &i
         if (name == "la_segs") return put(H.segs);
         if (name == "la_rec") return put(std::vector<int>(H.rec.begin(), H.rec.end()));
         if (name == "la_old") return put(std::vector<int>(H.old.begin(), H.old.end()));
+    }
+    if (name.rfind("strip_", 0) == 0) {  // the strip layout (strip_layout.h), built on request; empty where it does not apply
+        StripHost H;
+        if (!strip_build(P, H)) return put(std::vector<int>{});
+        if (name == "strip_dim") return put(std::vector<int>{H.w, H.rows, ST_STEPS, ST_WIN});
+        if (name == "strip_first") return put(H.first);
+        if (name == "strip_perm") return put(H.perm);
+        if (name == "strip_rows") return put(std::vector<int>(H.rows_sorted.begin(), H.rows_sorted.end()));
+        if (name == "strip_rows_at") return put(std::vector<int>(H.rows_at.begin(), H.rows_at.end()));
+        if (name == "strip_rec") return put(std::vector<int>(H.rec.begin(), H.rec.end()));
     }
     if (name.rfind("lc_", 0) == 0) ensure_lc(const_cast<Plan &>(P));
     if (name == "lc_tab") return put(P.lc_tab);

@@ -90,6 +90,8 @@ struct alignas(sizeof(T) * N) Vec {
 // ---------------------------------------------------------------------------
 // Vector permutations (utils_cuda.h:858-876 levelset_reordering_vecb/vecx,
 // fused with the RHS interleave, the precision cast and the sentinel reset).
+// perm[p] is the original row of position p, or -1 at a padding position of
+// the strip order (zero in, nothing out).
 // ---------------------------------------------------------------------------
 template <typename VT, int K>
 __global__ void k_gather(const double *__restrict__ b, int ld, int k, const int *__restrict__ perm, int n,
@@ -98,7 +100,8 @@ __global__ void k_gather(const double *__restrict__ b, int ld, int k, const int 
     long long total = (long long)n * K;
     for (; t < total; t += (long long)gridDim.x * blockDim.x) {
         int p = (int)(t / K), c = (int)(t % K);
-        double v = c < k ? b[(long long)c * ld + perm[p]] : 0.0;
+        const int i = perm[p];
+        double v = c < k && i >= 0 ? b[(long long)c * ld + i] : 0.0;
         out[t] = (VT)v;
     }
 }
@@ -112,7 +115,8 @@ __global__ void k_scatter_reset(VT *__restrict__ xw, const int *__restrict__ per
     for (; t < total; t += (long long)gridDim.x * blockDim.x) {
         int p = (int)(t / K), c = (int)(t % K);
         VT v = xw[t];
-        if (c < k) x[(long long)c * ld + perm[p]] = (double)v;
+        const int i = perm[p];
+        if (c < k && i >= 0) x[(long long)c * ld + i] = (double)v;
         xw[t] = Sent<VT>::value();
     }
 }
@@ -127,7 +131,8 @@ __global__ void k_gather_cols(const double *const *__restrict__ cols, int k, con
     const long long total = (long long)n * K;
     for (; t < total; t += (long long)gridDim.x * blockDim.x) {
         const int p = (int)(t / K), c = (int)(t % K);
-        out[t] = c < k ? (VT)cols[c][perm[p]] : VT(0);
+        const int i = perm[p];
+        out[t] = c < k && i >= 0 ? (VT)cols[c][i] : VT(0);
     }
 }
 
@@ -140,7 +145,8 @@ __global__ void k_scatter_cols(VT *__restrict__ xw, const int *__restrict__ perm
     for (; t < total; t += (long long)gridDim.x * blockDim.x) {
         const int p = (int)(t / K), c = (int)(t % K);
         const VT v = xw[t];
-        if (c < k) cols[c][perm[p]] = (double)v;
+        const int i = perm[p];
+        if (c < k && i >= 0) cols[c][i] = (double)v;
         xw[t] = Sent<VT>::value();
     }
 }
@@ -274,7 +280,7 @@ __global__ void __launch_bounds__(256) k_gather_grp(const double *__restrict__ b
     const long long i = perm[p];
     long long r = i;
     int f = 0;
-    if (grp.tab) {
+    if (grp.tab && i >= 0) {
         f = grp.seg[i];
         r = i - grp.off[f];
     }
@@ -285,7 +291,7 @@ __global__ void __launch_bounds__(256) k_gather_grp(const double *__restrict__ b
         for (int j = 0; j < GL; ++j) {
             const int c = (g0 + a) * GL + j;
             double t = 0.0;
-            if (c < k) {
+            if (c < k && i >= 0) {
                 if (grp.tab) {
                     const double *src = grp.tab[(long long)c * grp.F + f];
                     if (src) t = src[r];
@@ -329,7 +335,7 @@ __global__ void __launch_bounds__(256) k_scatter_grp(VT *__restrict__ xw, const 
     const long long i = perm[p];
     long long r = i;
     int f = 0;
-    if (grp.tab) {
+    if (grp.tab && i >= 0) {
         f = grp.seg[i];
         r = i - grp.off[f];
     }
@@ -352,7 +358,7 @@ __global__ void __launch_bounds__(256) k_scatter_grp(VT *__restrict__ xw, const 
 #pragma unroll
         for (int j = 0; j < GL; ++j) {
             const int c = (g0 + a) * GL + j;
-            if (c >= k) continue;
+            if (c >= k || i < 0) continue;
             const double t = (double)w[a].v[j];
             if (grp.tab) {
                 double *dst = const_cast<double *>(grp.tab[(long long)c * grp.F + f]);
@@ -905,7 +911,8 @@ __global__ void k_scatter64(const double *__restrict__ x64, const int *__restric
     long long total = (long long)n * K;
     for (; t < total; t += (long long)gridDim.x * blockDim.x) {
         int p = (int)(t / K), c = (int)(t % K);
-        if (c < k) x[(long long)c * ld + perm[p]] = x64[t];
+        const int i = perm[p];
+        if (c < k && i >= 0) x[(long long)c * ld + i] = x64[t];
     }
 }
 
@@ -917,7 +924,8 @@ __global__ void k_scatter64_cols(const double *__restrict__ x64, const int *__re
     const long long total = (long long)n * K;
     for (; t < total; t += (long long)gridDim.x * blockDim.x) {
         const int p = (int)(t / K), c = (int)(t % K);
-        if (c < k) cols[c][perm[p]] = x64[t];
+        const int i = perm[p];
+        if (c < k && i >= 0) cols[c][i] = x64[t];
     }
 }
 

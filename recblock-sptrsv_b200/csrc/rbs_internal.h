@@ -213,6 +213,21 @@ struct LaHost {
     bulk_vector<uint32_t> rec;  // FP64 records (the FP32 ones are made from them on the device)
     bulk_vector<int> old;       // positions of the old entries
 };
+// Strip layout of the whole matrix (strip_layout.h): records of every chunk,
+// strips' first chunks, and the strip order of the rows.  Derived from the
+// processing-order CSR when a plan's device state is built; not part of a
+// saved plan.
+struct StripHost {
+    bool ok = false;
+    int w = 0, rows = 0;        // slots per row, positions (padding included)
+    std::vector<int> first;     // first chunk of every strip, and the end
+    std::vector<int> perm;      // position -> processing position (-1: padding)
+    int published = 0;                   // rows whose values go through the exchange
+    bulk_vector<int> rows_sorted;        // per chunk its original rows ascending (-1 last)
+    bulk_vector<unsigned char> rows_at;  // and the position in the chunk of each
+    bulk_vector<uint32_t> rec;  // FP64 records (the FP32 ones are made from them on the device)
+};
+
 struct Plan {
     int n = 0, nnz = 0, lv = 0, sub = 0, nlevel = 0, sum_block = 0, step = 0;
     rbs_options opt{};
@@ -247,11 +262,12 @@ struct Plan {
     // chunk, chunks, ring offset of the first chunk)
     bulk_vector<uint32_t> lc_rec64, lc_rec32;
     std::vector<int> lc_tab, lc_segs;
-    // Plans that run on the look-ahead kernel leave the level-chunk records
+    // Plans that run on a whole-matrix kernel leave the level-chunk records
     // out until they are asked for (ensure_lc); the look-ahead layout is kept
     // here from the analysis to the upload.
     bool lc_deferred = false;
     std::shared_ptr<LaHost> la;
+    std::shared_ptr<StripHost> strip;  // the same for the strip kernel
     // original-row offsets of independent systems (batched plans); empty
     // for a single system
     std::vector<int> seg_rows;
@@ -322,6 +338,10 @@ int analyse_after_levels(Plan &P, int n, int nnz, int substitution, int lv, cons
 bool wants_la(const Plan &P);
 // analysis.cpp: builds the level-chunk records a plan left out
 void ensure_lc(Plan &P);
+// analysis.cpp: whether strips are worth trying for the plan's whole walk
+bool wants_strips(const Plan &P);
+// strip_build.h; false: the structure does not suit the kernel
+bool strip_build(const Plan &P, StripHost &H);
 // la_build.h; false: the structure does not suit the kernel
 bool la_build(const Plan &P, LaHost &H);
 

@@ -19,6 +19,7 @@
 #include "level_ca.cuh"
 #include "level_lc.cuh"
 #include "level_la.cuh"
+#include "level_strip.cuh"
 #include "rbs_internal.h"
 
 namespace rbs {
@@ -44,6 +45,7 @@ struct DeviceState {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_in = nullptr;  // the default stream's work before a solve on the plan's own stream
     // plan pools
     int *rp = nullptr, *col = nullptr, *lvl = nullptr, *map = nullptr, *rows = nullptr, *perm = nullptr;
     int *ipos = nullptr;  // original row -> processing position (inverse of perm)
@@ -78,6 +80,22 @@ struct DeviceState {
     uint32_t *la_rec64 = nullptr, *la_rec32 = nullptr;
     int *la_old = nullptr;
     int la_nseg = 0, la_gather = 0;
+    // strip layout of the whole matrix (level_strip.cuh); with it perm, ipos
+    // and the full CSR are in strip order
+    bool strip = false;
+    int strip_w = 0, strip_n = 0, strip_pub = 0;
+    int *strip_first = nullptr, *strip_ticket = nullptr, *strip_rows = nullptr;
+    unsigned char *strip_at = nullptr;
+    // two exchange vectors per precision, used in turn: a walk clears the
+    // other one's numbers; columns beyond its own that still hold values
+    template <typename VT> struct Exchange {
+        VT *buf[2] = {nullptr, nullptr};
+        int cur = 0, dirty[2] = {0, 0};
+    };
+    Exchange<double> ex64;
+    Exchange<float> ex32;
+    uint32_t *strip_rec64 = nullptr, *strip_rec32 = nullptr;
+    int wn = 0;  // positions of the work vectors (rows, or more with padding)
     int *la_queue = nullptr;  // one segment counter per column
     cudaStream_t side = nullptr;                         // L2 prefetch stream; moves of the overlapped walk
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -197,6 +215,12 @@ void free_work(DeviceState &D) {
     cudaFree(D.xw32);
     D.bw64 = D.xw64 = D.b64keep = D.x64acc = nullptr;
     D.bw32 = D.xw32 = nullptr;
+    for (int i = 0; i < 2; ++i) {
+        cudaFree(D.ex64.buf[i]);
+        cudaFree(D.ex32.buf[i]);
+    }
+    D.ex64 = {};
+    D.ex32 = {};
     for (auto &kv : D.desc_cache) cudaFree(kv.second);
     D.desc_cache.clear();
     for (auto &kv : D.ell_cache) cudaFree(kv.second);
@@ -230,15 +254,22 @@ int ensure_work(Plan &P, int K, std::string &err) {
     D.work_bytes = 0;
     D.kcap = 0;
     const long long before = D.bytes;
-    const size_t cnt = (size_t)P.n * K;
+    const size_t cnt = (size_t)D.wn * K;
     auto undo = [&](int rc) {
         free_work(D);
         D.bytes = before;
         return rc;
     };
     int rc;
-    if ((rc = alloc(D, D.bw64, cnt, err))) return undo(rc);
-    if ((rc = alloc(D, D.xw64, cnt, err))) return undo(rc);
+    if (D.strip) {  // FP64 walks run on the caller's vectors
+        for (int i = 0; i < 2; ++i) {
+            if ((rc = alloc(D, D.ex64.buf[i], (size_t)D.strip_pub * (K + 1), err))) return undo(rc);
+            if (D.mixed && (rc = alloc(D, D.ex32.buf[i], (size_t)D.strip_pub * (K + 1), err))) return undo(rc);
+        }
+    } else {
+        if ((rc = alloc(D, D.bw64, cnt, err))) return undo(rc);
+        if ((rc = alloc(D, D.xw64, cnt, err))) return undo(rc);
+    }
     if (D.mixed) {
         if ((rc = alloc(D, D.b64keep, cnt, err))) return undo(rc);
         if ((rc = alloc(D, D.x64acc, cnt, err))) return undo(rc);
@@ -247,11 +278,19 @@ int ensure_work(Plan &P, int K, std::string &err) {
     }
     if ((rc = alloc(D, D.band_maps, D.band_maps1 * K, err))) return undo(rc);
     if ((rc = alloc(D, D.band_states, D.band_states1 * K, err))) return undo(rc);
-    k_fill<double><<<grid_for((long long)cnt, 256, D.num_sms), 256, 0, D.stream>>>(D.xw64, (long long)cnt,
-                                                                                    sent64_host());
-    if (D.mixed)
-        k_fill<float><<<grid_for((long long)cnt, 256, D.num_sms), 256, 0, D.stream>>>(D.xw32, (long long)cnt,
-                                                                                       sent32_host());
+    if (D.strip) {
+        if (D.mixed) {  // padding positions stay zero in every right-hand side
+            CK(cudaMemsetAsync(D.b64keep, 0, cnt * sizeof(double), D.stream));
+            CK(cudaMemsetAsync(D.bw32, 0, cnt * sizeof(float), D.stream));
+        }
+        D.ex64.dirty[0] = D.ex64.dirty[1] = D.ex32.dirty[0] = D.ex32.dirty[1] = K + 1;  // filled before use
+    } else {
+        k_fill<double><<<grid_for((long long)cnt, 256, D.num_sms), 256, 0, D.stream>>>(D.xw64, (long long)cnt,
+                                                                                        sent64_host());
+        if (D.mixed)
+            k_fill<float><<<grid_for((long long)cnt, 256, D.num_sms), 256, 0, D.stream>>>(D.xw32, (long long)cnt,
+                                                                                           sent32_host());
+    }
     D.xw_dirty64 = D.xw_dirty32 = false;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -273,6 +312,8 @@ template <> struct Pools<double> {
     static const double *cav(const DeviceState &D) { return D.ca_val; }
     static const unsigned char *lcrec(const DeviceState &D) { return reinterpret_cast<const unsigned char *>(D.lc_rec64); }
     static const uint32_t *larec(const DeviceState &D) { return D.la_rec64; }
+    static const uint32_t *striprec(const DeviceState &D) { return D.strip_rec64; }
+    static DeviceState::Exchange<double> &ex(DeviceState &D) { return D.ex64; }
     static double *bw(const DeviceState &D) { return D.bw64; }
     static double *xw(const DeviceState &D) { return D.xw64; }
     static bool &dirty(DeviceState &D) { return D.xw_dirty64; }
@@ -287,6 +328,8 @@ template <> struct Pools<float> {
     static const float *cav(const DeviceState &D) { return D.ca_val32; }
     static const unsigned char *lcrec(const DeviceState &D) { return reinterpret_cast<const unsigned char *>(D.lc_rec32); }
     static const uint32_t *larec(const DeviceState &D) { return D.la_rec32; }
+    static const uint32_t *striprec(const DeviceState &D) { return D.strip_rec32; }
+    static DeviceState::Exchange<float> &ex(DeviceState &D) { return D.ex32; }
     static float *bw(const DeviceState &D) { return D.bw32; }
     static float *xw(const DeviceState &D) { return D.xw32; }
     static bool &dirty(DeviceState &D) { return D.xw_dirty32; }
@@ -415,6 +458,14 @@ template <typename VT> int ca_group(const ExecBlock &B, int K) {
     return G;
 }
 
+// Columns per CTA of the strip kernel: one while every strip of every column
+// has a CTA on the GPU at once, two otherwise (1M-row grid, 32 columns: one
+// 563, two 505, four 562 us).
+template <typename VT> int strip_group(const DeviceState &D, int cols) {
+    const int smem = D.strip_w == 2 ? st_smem<VT, 2, 1, true>() : st_smem<VT, 4, 1, true>();
+    return cols == 1 || (long long)D.strip_n * cols <= (long long)D.num_sms * (D.smem_sm / (smem + D.smem_reserved)) ? 1 : 2;
+}
+
 // Layout of a K-column solve's work vectors: 0 = row-interleaved (entry
 // (p, c) at p*K + c), G > 0 = grouped by column groups of G (group c/G's
 // rows contiguous, G values each), taken when every triangle is a staged
@@ -423,6 +474,7 @@ template <typename VT> int ca_group(const ExecBlock &B, int K) {
 template <typename VT> int plan_group(const Plan &P, int K) {
     if (K == 1) return 0;
     if (P.dev->la) return 1;  // the look-ahead kernel: one CTA per column, columns contiguous
+    if (P.dev->strip) return strip_group<VT>(*P.dev, K);
     int G = 2;
     for (const ExecBlock &B : P.blocks) {
         if (!B.tri || B.nnz == B.m) continue;
@@ -770,6 +822,10 @@ int move_reserve(const DeviceState &D, size_t ca_min) {
     return (int)need;
 }
 
+// Poll budget of the whole-matrix kernels: they also wait for their own
+// copies, where a plan's smaller spin_limit would give up on ordinary latency.
+long long wait_limit(const Plan &P) { return std::max(P.opt.spin_limit, 1LL << 20); }
+
 // Whole-matrix walk of the look-ahead kernel: one launch, K columns side by side.
 template <typename VT, int Q>
 int launch_la_q(DeviceState &D, const LaArgs<VT> &a, int K, std::string &err) {
@@ -799,7 +855,7 @@ int launch_la(Plan &P, int K, std::string &err) {
     a.n = P.n;
     a.queue = D.la_queue;
     a.status = D.status;
-    a.limit = P.opt.spin_limit;
+    a.limit = wait_limit(P);
     a.d = D.la_dim;
     a.slots = a.d.slots(sizeof(VT));
     a.gather = D.la_gather;
@@ -809,16 +865,110 @@ int launch_la(Plan &P, int K, std::string &err) {
                         : launch_la_q<VT, 12>(D, a, K, err);
 }
 
+// Whole-matrix walk of the strip kernel: one CTA per strip and group of G columns.
+template <typename VT, int W, int G, bool IO>
+int launch_strip_wg(DeviceState &D, const StripArgs<VT> &a, int groups, std::string &err) {
+    constexpr int smem = st_smem<VT, W, G, IO>();
+    static std::atomic<unsigned long long> attr{0};
+    if (!attr_done(attr)) {
+        CK(cudaFuncSetAttribute(k_tri_strip<VT, W, G, IO>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        attr_mark(attr);
+    }
+    k_tri_strip<VT, W, G, IO><<<dim3((unsigned)a.nstrip, (unsigned)groups), 96, smem, D.stream>>>(a);
+    CK(cudaGetLastError());
+    return RBS_OK;
+}
+
+// The arguments that both kinds of walk share, for `cols` columns in groups
+// of G: the exchange vectors change places, and one that still holds values
+// (of a wider walk, or a failed one) is cleared first.
+template <typename VT>
+int strip_args(Plan &P, StripArgs<VT> &a, int cols, int G, std::string &err) {
+    DeviceState &D = *P.dev;
+    auto &X = Pools<VT>::ex(D);
+    const int groups = (cols + G - 1) / G, used = groups * G;
+    a.rec = reinterpret_cast<const unsigned char *>(Pools<VT>::striprec(D));
+    a.first = D.strip_first;
+    a.nstrip = D.strip_n;
+    a.rows = D.strip_rows;
+    a.rows_at = D.strip_at;
+    a.published = D.strip_pub;
+    a.ticket = D.strip_ticket;
+    a.status = D.status;
+    a.limit = wait_limit(P);
+    const int other = X.cur ^ 1;
+    for (int i = 0; i < 2; ++i)
+        if (X.dirty[i] > (i == X.cur ? 0 : used)) {
+            const long long cnt = (long long)D.strip_pub * (D.kcap + 1);
+            k_fill<VT><<<grid_for(cnt, 256, D.num_sms), 256, 0, D.stream>>>(X.buf[i], cnt, Pools<VT>::sent());
+            X.dirty[i] = 0;
+        }
+    a.ex = X.buf[X.cur];
+    a.ex_next = X.buf[other];
+    X.dirty[X.cur] = used;
+    X.dirty[other] = 0;
+    X.cur = other;
+    CK(cudaMemsetAsync(D.strip_ticket, 0, sizeof(int) * (size_t)groups, D.stream));
+    return RBS_OK;
+}
+
+// Walk on the work vectors in strip order (the FP32 sweeps of refinement).
+template <typename VT>
+int launch_strip(Plan &P, int K, std::string &err) {
+    DeviceState &D = *P.dev;
+    const int G = K == 1 ? 1 : strip_group<VT>(D, K), groups = K / G;
+    StripArgs<VT> a{};
+    int rc = strip_args<VT>(P, a, K, G, err);
+    if (rc) return rc;
+    a.b = Pools<VT>::bw(D);
+    a.x = Pools<VT>::xw(D);
+    a.gstride = (long long)D.wn * G;
+    if (D.strip_w == 2)
+        return G == 1 ? launch_strip_wg<VT, 2, 1, false>(D, a, groups, err) : launch_strip_wg<VT, 2, 2, false>(D, a, groups, err);
+    return G == 1 ? launch_strip_wg<VT, 4, 1, false>(D, a, groups, err) : launch_strip_wg<VT, 4, 2, false>(D, a, groups, err);
+}
+
+// Walk on the caller's columns (b + c * ld and x + c * ld, or the tables).
+template <typename VT>
+int solve_strip(Plan &P, const double *b, double *x, const double *const *bcols, double *const *xcols, int k, int ld,
+                std::string &err) {
+    DeviceState &D = *P.dev;
+    const int G = strip_group<VT>(D, k), groups = (k + G - 1) / G;
+    if (D.profile)
+        for (const ExecBlock &B : P.blocks) {
+            CK(cudaEventRecord(D.bev[2 * B.index], D.stream));
+            if (B.index) CK(cudaEventRecord(D.bev[2 * B.index + 1], D.stream));
+        }
+    StripArgs<VT> a{};
+    int rc = strip_args<VT>(P, a, k, G, err);
+    if (rc) return rc;
+    a.b64 = b;
+    a.x64 = x;
+    a.bcols = bcols;
+    a.xcols = xcols;
+    a.ld = ld;
+    a.k = k;
+    if (D.strip_w == 2)
+        rc = G == 1 ? launch_strip_wg<VT, 2, 1, true>(D, a, groups, err) : launch_strip_wg<VT, 2, 2, true>(D, a, groups, err);
+    else
+        rc = G == 1 ? launch_strip_wg<VT, 4, 1, true>(D, a, groups, err) : launch_strip_wg<VT, 4, 2, true>(D, a, groups, err);
+    if (rc) return rc;
+    if (D.profile) CK(cudaEventRecord(D.bev[1], D.stream));
+    return RBS_OK;
+}
+
 // One pass over all blocks: triangles solve into xw, squares update bw.
 template <typename VT, int K>
 int launch_blocks(Plan &P, std::string &err, bool io = false) {
     DeviceState &D = *P.dev;
     cudaStream_t st = D.stream;
-    if (D.la) {  // profiled walks report the whole launch as the first block's time
+    if (D.la || D.strip) {  // profiled walks report the whole launch as the first block's time
         for (const ExecBlock &B : P.blocks) {
             if (D.profile) CK(cudaEventRecord(D.bev[2 * B.index], st));
             if (B.index == 0) {
-                const int rc = launch_la<VT>(P, K, err);
+                int rc = RBS_ERR_UNSUPPORTED;
+                if (D.la) rc = launch_la<VT>(P, K, err);
+                else if constexpr (sizeof(VT) == 4) rc = launch_strip<VT>(P, K, err);  // FP64 walks run on the caller's vectors
                 if (rc) return rc;
             }
             if (D.profile) CK(cudaEventRecord(D.bev[2 * B.index + 1], st));
@@ -1072,7 +1222,7 @@ int launch_blocks(Plan &P, std::string &err, bool io = false) {
 // vector for its sentinel (the sync-free kernels), with the kernel choice
 // of launch_blocks.
 bool walk_polls(const Plan &P, int K) {
-    if (P.dev->la) return false;
+    if (P.dev->la || P.dev->strip) return false;
     for (const ExecBlock &B : P.blocks) {
         if (!B.tri) continue;
         if (B.kernel == RBS_K_SYNCFREE) return true;
@@ -1087,13 +1237,13 @@ template <typename VT, int K>
 int run_blocks(Plan &P, std::string &err, bool io = false) {
     DeviceState &D = *P.dev;
     if (!io && Pools<VT>::dirty(D) && walk_polls(P, K)) {  // the sync-free kernels poll x for the sentinel
-        const long long cnt = (long long)P.n * D.kcap;
+        const long long cnt = (long long)D.wn * D.kcap;
         k_fill<VT><<<grid_for(cnt, 256, D.num_sms), 256, 0, D.stream>>>(Pools<VT>::xw(D), cnt, Pools<VT>::sent());
         Pools<VT>::dirty(D) = false;
     }
     // per-block timing needs real event timestamps, which captured event
     // records are not: profiled solves launch eagerly
-    if (!D.use_graphs || D.profile || D.la) return launch_blocks<VT, K>(P, err, io);
+    if (!D.use_graphs || D.profile || D.la || D.strip) return launch_blocks<VT, K>(P, err, io);
     const long long key = (long long)K * 8 + (sizeof(VT) == 8 ? 0 : 2) + (io ? 4 : 0);
     auto it = D.graphs.find(key);
     if (it != D.graphs.end()) {
@@ -1146,16 +1296,16 @@ void gather_in(DeviceState &D, int n, const double *b, int ld, const double *con
                VT2 *out2, int GL, GroupCols grp = GroupCols{}) {
     const int tgrid = std::max(1, (int)std::min<long long>(((long long)n + TP_ROWS - 1) / TP_ROWS, (long long)D.num_sms * 8));
     if (GL) {
-        gather_grp<VT, VT2, K>(D, D.stream, n, b, ld, cols, k, out, out2, GL, grp, 0, n);
+        gather_grp<VT, VT2, K>(D, D.stream, D.wn, b, ld, cols, k, out, out2, GL, grp, 0, D.wn);
     } else if (K >= 8 || grp.tab) {
         k_gather_t<VT, VT2, K><<<tgrid, 256, 0, D.stream>>>(b, ld, cols, k, D.ipos, n, out, out2, grp);
     } else {
-        const int grid = grid_for((long long)n * K, 256, D.num_sms);
-        if (cols) k_gather_cols<VT, K><<<grid, 256, 0, D.stream>>>(cols, k, D.perm, n, out);
-        else k_gather<VT, K><<<grid, 256, 0, D.stream>>>(b, ld, k, D.perm, n, out);
+        const int grid = grid_for((long long)D.wn * K, 256, D.num_sms);
+        if (cols) k_gather_cols<VT, K><<<grid, 256, 0, D.stream>>>(cols, k, D.perm, D.wn, out);
+        else k_gather<VT, K><<<grid, 256, 0, D.stream>>>(b, ld, k, D.perm, D.wn, out);
         if (out2) {
-            if (cols) k_gather_cols<VT2, K><<<grid, 256, 0, D.stream>>>(cols, k, D.perm, n, out2);
-            else k_gather<VT2, K><<<grid, 256, 0, D.stream>>>(b, ld, k, D.perm, n, out2);
+            if (cols) k_gather_cols<VT2, K><<<grid, 256, 0, D.stream>>>(cols, k, D.perm, D.wn, out2);
+            else k_gather<VT2, K><<<grid, 256, 0, D.stream>>>(b, ld, k, D.perm, D.wn, out2);
         }
     }
 }
@@ -1167,18 +1317,18 @@ void scatter_out(DeviceState &D, int n, VT *xw, int k, double *x, int ld, double
                  GroupCols grp = GroupCols{}) {
     const int tgrid = std::max(1, (int)std::min<long long>(((long long)n + TP_ROWS - 1) / TP_ROWS, (long long)D.num_sms * 8));
     if (GL) {
-        scatter_grp<VT, K, RESET>(D, D.stream, n, xw, k, x, ld, cols, GL, grp, 0, n);
+        scatter_grp<VT, K, RESET>(D, D.stream, D.wn, xw, k, x, ld, cols, GL, grp, 0, D.wn);
     } else if (K >= 8 || grp.tab) {
         k_scatter_t<VT, K, RESET><<<tgrid, 256, 0, D.stream>>>(xw, D.ipos, n, k, x, ld, cols, grp);
     } else {
-        const int grid = grid_for((long long)n * K, 256, D.num_sms);
+        const int grid = grid_for((long long)D.wn * K, 256, D.num_sms);
         if constexpr (RESET) {
-            if (cols) k_scatter_cols<VT, K><<<grid, 256, 0, D.stream>>>(xw, D.perm, n, k, cols);
-            else k_scatter_reset<VT, K><<<grid, 256, 0, D.stream>>>(xw, D.perm, n, k, x, ld);
+            if (cols) k_scatter_cols<VT, K><<<grid, 256, 0, D.stream>>>(xw, D.perm, D.wn, k, cols);
+            else k_scatter_reset<VT, K><<<grid, 256, 0, D.stream>>>(xw, D.perm, D.wn, k, x, ld);
         } else {
             static_assert(RESET || std::is_same<VT, double>::value, "FP64 accumulator only");
-            if (cols) k_scatter64_cols<K><<<grid, 256, 0, D.stream>>>(xw, D.perm, n, k, cols);
-            else k_scatter64<K><<<grid, 256, 0, D.stream>>>(xw, D.perm, n, k, x, ld);
+            if (cols) k_scatter64_cols<K><<<grid, 256, 0, D.stream>>>(xw, D.perm, D.wn, k, cols);
+            else k_scatter64<K><<<grid, 256, 0, D.stream>>>(xw, D.perm, D.wn, k, x, ld);
         }
     }
 }
@@ -1189,6 +1339,7 @@ void scatter_out(DeviceState &D, int n, VT *xw, int k, double *x, int ld, double
 template <int K>
 int solve_fp64(Plan &P, const double *b, double *x, int k, int ld, std::string &err) {
     DeviceState &D = *P.dev;
+    if (D.strip) return solve_strip<double>(P, b, x, nullptr, nullptr, k, ld, err);
     const int GL = plan_group<double>(P, K);
     if (K > 1 && GL && !D.la) {
         int rc = ensure_io_rows(P, err);
@@ -1210,6 +1361,7 @@ int solve_fp64(Plan &P, const double *b, double *x, int k, int ld, std::string &
 template <int K>
 int solve_fp32(Plan &P, const double *b, double *x, int k, int ld, std::string &err) {
     DeviceState &D = *P.dev;
+    if (D.strip) return solve_strip<float>(P, b, x, nullptr, nullptr, k, ld, err);
     const int GL = plan_group<float>(P, K);
     if (K > 1 && GL && !D.la) {
         int rc = ensure_io_rows(P, err);
@@ -1239,12 +1391,12 @@ void mixed_update(Plan &P, int first) {
     DeviceState &D = *P.dev;
     const int GL = plan_group<float>(P, K);
     if (GL) {
-        const dim3 grid((unsigned)std::max(1, std::min((P.n + 255) / 256, 2 * D.num_sms)), K);
-        if (GL == 1) k_update_grp<K, 1><<<grid, 256, 0, D.stream>>>(D.x64acc, D.xw32, P.n, first, D.norms);
-        else k_update_grp<K, 2><<<grid, 256, 0, D.stream>>>(D.x64acc, D.xw32, P.n, first, D.norms);
+        const dim3 grid((unsigned)std::max(1, std::min((D.wn + 255) / 256, 2 * D.num_sms)), K);
+        if (GL == 1) k_update_grp<K, 1><<<grid, 256, 0, D.stream>>>(D.x64acc, D.xw32, D.wn, first, D.norms);
+        else k_update_grp<K, 2><<<grid, 256, 0, D.stream>>>(D.x64acc, D.xw32, D.wn, first, D.norms);
         return;
     }
-    k_update<K><<<grid_for((long long)P.n * K, 256, D.num_sms), 256, 0, D.stream>>>(D.x64acc, D.xw32, P.n, first,
+    k_update<K><<<grid_for((long long)D.wn * K, 256, D.num_sms), 256, 0, D.stream>>>(D.x64acc, D.xw32, D.wn, first,
                                                                                       D.norms);
 }
 
@@ -1263,7 +1415,7 @@ int mixed_first(Plan &P, std::string &err) {
 template <int K>
 int mixed_step(Plan &P, std::string &err) {
     DeviceState &D = *P.dev;
-    const int n = P.n;
+    const int n = D.wn;
     const int G = P.nnz / std::max(1, n) < 6 ? 4 : 8;
     const int GL = plan_group<float>(P, K);
     if (GL == 1)
@@ -1345,6 +1497,9 @@ int batch_start_k(Plan &P, const double *const *bcols, double *const *xcols, int
     DeviceState &D = *P.dev;
     const int n = P.n;
     int rc;
+    if (D.strip && prec != RBS_PREC_MIXED)
+        return prec == RBS_PREC_FP64 ? solve_strip<double>(P, nullptr, nullptr, bcols, xcols, k, n, err)
+                                     : solve_strip<float>(P, nullptr, nullptr, bcols, xcols, k, n, err);
     if (prec == RBS_PREC_FP64) {
         const int GL = plan_group<double>(P, K);
         gather_in<double, double, K>(D, n, nullptr, n, bcols, k, D.bw64, nullptr, GL, gb);
@@ -1496,6 +1651,68 @@ int upload_la(Plan &P, std::string &err) {
     return RBS_OK;
 }
 
+// Builds and uploads the strip layout (D.strip stays false where the
+// structure does not suit it): records, the strip order, and, for mixed
+// precision, the full CSR in that order (padding rows empty).
+int upload_strips(Plan &P, std::string &err) {
+    DeviceState &D = *P.dev;
+    if (!P.strip) {
+        P.strip = std::make_shared<StripHost>();
+        strip_build(P, *P.strip);
+    }
+    if (!P.strip->ok) return RBS_OK;
+    const StripHost &H = *P.strip;
+    int rc;
+    std::vector<int> perm((size_t)H.rows), ipos((size_t)P.n), pos((size_t)P.n);
+    for (int q = 0; q < H.rows; ++q) {
+        const int p = H.perm[(size_t)q];
+        perm[(size_t)q] = p < 0 ? -1 : P.perm[(size_t)p];
+        if (p < 0) continue;
+        pos[(size_t)p] = q;
+        ipos[(size_t)P.perm[(size_t)p]] = q;
+    }
+    if ((rc = upload(D, D.perm, perm, err)) || (rc = upload(D, D.ipos, ipos, err)) ||
+        (rc = upload(D, D.strip_first, H.first, err)) || (rc = upload(D, D.strip_rec64, H.rec, err)) ||
+        (rc = upload(D, D.strip_rows, H.rows_sorted, err)) || (rc = upload(D, D.strip_at, H.rows_at, err)) ||
+        (rc = alloc(D, D.strip_ticket, 128, err)))
+        return rc;
+    if (D.mixed) {
+        const int nch = H.first.back();
+        if ((rc = alloc(D, D.strip_rec32, (size_t)nch * st_rec_bytes(H.w, 4) / 4, err))) return rc;
+        k_strip_rec32<<<(unsigned)nch, 128, 0, D.stream>>>(H.w, reinterpret_cast<const unsigned char *>(D.strip_rec64),
+                                                           reinterpret_cast<unsigned char *>(D.strip_rec32));
+        CK(cudaGetLastError());
+        std::vector<int> rp((size_t)H.rows + 1, 0);
+        for (int q = 0; q < H.rows; ++q) {
+            const int p = H.perm[(size_t)q];
+            rp[(size_t)q + 1] = rp[(size_t)q] + (p < 0 ? 0 : P.full_rp[(size_t)p + 1] - P.full_rp[(size_t)p]);
+        }
+        bulk_vector<int> ci(P.full_col.size());
+        bulk_vector<double> va(P.full_val.size());
+        parallel_for((size_t)H.rows / ST_ROWS, [&](size_t c) {
+            for (size_t q = c * ST_ROWS; q < (c + 1) * ST_ROWS; ++q) {
+                const int p = H.perm[q];
+                if (p < 0) continue;
+                int d = rp[q];
+                for (int k = P.full_rp[(size_t)p]; k < P.full_rp[(size_t)p + 1]; ++k, ++d) {
+                    ci[(size_t)d] = pos[(size_t)P.full_col[(size_t)k]];
+                    va[(size_t)d] = P.full_val[(size_t)k];
+                }
+            }
+        });
+        if ((rc = upload(D, D.full_rp, rp, err)) || (rc = upload(D, D.full_col, ci, err)) ||
+            (rc = upload(D, D.full_val, va, err)))
+            return rc;
+    }
+    D.strip_w = H.w;
+    D.strip_n = (int)H.first.size() - 1;
+    D.strip_pub = std::max(1, H.published);
+    D.wn = H.rows;
+    D.strip = true;
+    P.strip.reset();
+    return RBS_OK;
+}
+
 // The blocks' pools and per-kernel layouts (the block walk).
 int upload_blocks(Plan &P, std::string &err) {
     DeviceState &D = *P.dev;
@@ -1591,30 +1808,31 @@ int device_build(Plan &P, std::string &err) {
     D.own_stream = true;
     CK(cudaEventCreate(&D.ev0));
     CK(cudaEventCreate(&D.ev1));
+    CK(cudaEventCreateWithFlags(&D.ev_in, cudaEventDisableTiming));
     {
         const char *ng = std::getenv("RBS_NO_GRAPHS");
         D.use_graphs = !(ng && ng[0] == '1');
     }
     int rc;
-    if ((rc = upload(D, D.perm, P.perm, err))) return rc;
-    {
+    D.wn = P.n;
+    D.mixed = P.opt.mixed != 0;
+    if (wants_strips(P) && (rc = upload_strips(P, err))) return rc;
+    if (!D.strip) {
+        if ((rc = upload(D, D.perm, P.perm, err))) return rc;
         std::vector<int> ipos(P.perm.size());
         for (size_t p = 0; p < P.perm.size(); ++p) ipos[(size_t)P.perm[p]] = (int)p;
         if ((rc = upload(D, D.ipos, ipos, err))) return rc;
+        if ((rc = upload(D, D.inv, P.inv_diag, err))) return rc;
+        if (D.mixed) {
+            const auto i32 = to_f32(P.inv_diag);
+            if ((rc = upload(D, D.inv32, i32, err))) return rc;
+            if ((rc = upload(D, D.full_rp, P.full_rp, err))) return rc;
+            if ((rc = upload(D, D.full_col, P.full_col, err))) return rc;
+            if ((rc = upload(D, D.full_val, P.full_val, err))) return rc;
+        }
+        if (wants_la(P) && (rc = upload_la(P, err))) return rc;
     }
-    if ((rc = upload(D, D.inv, P.inv_diag, err))) return rc;
-    D.mixed = P.opt.mixed != 0;
-    if (D.mixed) {
-        const auto i32 = to_f32(P.inv_diag);
-        if ((rc = upload(D, D.inv32, i32, err))) return rc;
-        if ((rc = upload(D, D.full_rp, P.full_rp, err))) return rc;
-        if ((rc = upload(D, D.full_col, P.full_col, err))) return rc;
-        if ((rc = upload(D, D.full_val, P.full_val, err))) return rc;
-    }
-    if (wants_la(P)) {
-        if ((rc = upload_la(P, err))) return rc;
-    }
-    if (!D.la && (rc = upload_blocks(P, err))) return rc;
+    if (!D.la && !D.strip && (rc = upload_blocks(P, err))) return rc;
     {
         int prio_low = 0, prio_high = 0;
         CK(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
@@ -1882,6 +2100,12 @@ void device_free(Plan &P) {
     cudaFree(D.la_rec32);
     cudaFree(D.la_old);
     cudaFree(D.la_queue);
+    cudaFree(D.strip_first);
+    cudaFree(D.strip_ticket);
+    cudaFree(D.strip_rows);
+    cudaFree(D.strip_at);
+    cudaFree(D.strip_rec64);
+    cudaFree(D.strip_rec32);
     cudaFree(D.stage_b);
     cudaFree(D.stage_x);
     void *ptrs[] = {D.rp, D.col, D.lvl, D.map, D.rows, D.perm, D.ipos, D.val, D.inv, D.val32, D.inv32,
@@ -1892,6 +2116,7 @@ void device_free(Plan &P) {
     if (D.h_norms) cudaFreeHost(D.h_norms);
     if (D.ev0) cudaEventDestroy(D.ev0);
     if (D.ev1) cudaEventDestroy(D.ev1);
+    if (D.ev_in) cudaEventDestroy(D.ev_in);
     if (D.own_stream && D.stream) cudaStreamDestroy(D.stream);
     delete P.dev;
     P.dev = nullptr;
@@ -1927,7 +2152,7 @@ int device_sync(Plan &P, std::string &err) {
     if (*D.h_status & RBS_STATUS_TIMEOUT) {
         CK(cudaMemsetAsync(D.status, 0, sizeof(int), D.stream));
         // the solution work vectors may hold leftovers of the aborted solve
-        size_t cnt = (size_t)P.n * D.kcap;
+        size_t cnt = (size_t)D.wn * D.kcap;
         if (D.xw64)
             k_fill<double><<<grid_for((long long)cnt, 256, D.num_sms), 256, 0, D.stream>>>(
                 D.xw64, (long long)cnt, sent64_host());
@@ -1935,6 +2160,7 @@ int device_sync(Plan &P, std::string &err) {
             k_fill<float><<<grid_for((long long)cnt, 256, D.num_sms), 256, 0, D.stream>>>(
                 D.xw32, (long long)cnt, sent32_host());
         D.xw_dirty64 = D.xw_dirty32 = false;
+        D.ex64.dirty[0] = D.ex64.dirty[1] = D.ex32.dirty[0] = D.ex32.dirty[1] = D.kcap + 1;
         CK(cudaStreamSynchronize(D.stream));
         err = "a device wait exceeded its poll budget (dependency never produced)";
         return RBS_ERR_TIMEOUT;
@@ -1958,6 +2184,14 @@ int device_solve(Plan &P, const double *d_b, double *d_x, int k, int ld, int pre
     int iters = 0;
     double corr = 0;
     int rc = RBS_OK;
+    // On the plan's own stream, work already queued on the default stream
+    // (a caller filling b or x just before) comes first: the whole-matrix
+    // walks write the first solutions a few microseconds after their launch.
+    // While another stream's capture forbids the event, the solve goes ahead.
+    if (D.own_stream) {
+        if (cudaEventRecord(D.ev_in, cudaStreamLegacy) == cudaSuccess) CK(cudaStreamWaitEvent(D.stream, D.ev_in, 0));
+        else cudaGetLastError();
+    }
     CK(cudaEventRecord(D.ev0, D.stream));
     for (int c0 = 0; c0 < k && rc == RBS_OK; c0 += 128) {
         int kk = std::min(128, k - c0);
