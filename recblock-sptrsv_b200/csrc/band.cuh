@@ -11,7 +11,7 @@
 // consecutive rows (a chunk); a CTA scans its BAND_T chunk maps in shared
 // memory (Kogge-Stone) and publishes their total; the state entering the
 // CTA is its predecessors' totals applied in order to the zero state (one
-// W x W matrix-vector product each, no scan of maps needed); each thread
+// composed pairwise across the CTA's threads); each thread
 // applies the composition of its CTA's earlier chunks to that state and
 // replays its rows from there.  CTAs take their place in the chain from a
 // ticket, so every predecessor a CTA waits for is already running and
@@ -21,6 +21,10 @@
 // three launches once the CTAs scanned their own chunks.
 // Band coefficients are stored chunk-interleaved (row i of chunk j at
 // [(i*nch + j)*W]) so the threads of a warp read consecutive addresses.
+// When every triangle of a plan is such a chain and no row reaches further
+// back across them either, the whole matrix is one scan on the caller's own
+// vectors (1M rows of bandwidth 3: 195 -> 49 us; eight triangles and seven
+// squares in a row before).
 // For diagonally dominant rows every ||M_p||_inf <= 1, so composed maps stay
 // bounded and the scan is as stable as substitution.
 #pragma once
@@ -54,7 +58,8 @@ __device__ __forceinline__ void band_step_M(VT (&M)[W][W], VT (&c)[W], const VT 
     c[0] = c0;
 }
 
-// Chunks per CTA of the maps and replay passes (the CTA-level scan's width).
+// Chunks per CTA of the maps and replay passes (the CTA-level scan's width;
+// 512 with half the rows per chunk was slower on 1M rows: 57 against 49 us).
 constexpr int BAND_T = 256;
 
 __host__ __device__ constexpr int band_blocks(int nch) { return (nch + BAND_T - 1) / BAND_T; }
@@ -129,16 +134,19 @@ __device__ __forceinline__ void band_st_release(int *p, int v) {
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// One launch per triangle.  Several right-hand sides run side by side:
-// column c = blockIdx.y, with its own CTA totals at agg + c * nblk * (W*W+W)
-// and its own ticket and ready flags (flags: c * (nblk + 1), the ticket
-// first, then one flag per CTA; zeroed before the launch).  Waits are
-// bounded: after `limit` polls a CTA raises RBS_STATUS_TIMEOUT and goes on.
-template <typename VT, int W>
+// One launch per triangle (or per matrix).  Several right-hand sides run side
+// by side: column c = blockIdx.y, with its own CTA totals at agg + c * nblk *
+// (W*W+W) and its own ticket and ready flags (flags: c * (nblk + 1), the
+// ticket first, then one flag per CTA; zeroed before the launch).  Row p of
+// column c is element p * rs + c * cs of b and x: a work vector's, or the
+// caller's own (BT = double, rs = 1 or -1) where the rows are solved in the
+// caller's order or its reverse.  Waits are bounded: after `limit` polls a CTA
+// raises RBS_STATUS_TIMEOUT and goes on.
+template <typename VT, int W, typename BT>
 __global__ void __launch_bounds__(BAND_T) k_band_onepass(const VT *__restrict__ coef, const VT *__restrict__ inv,
-                                                         const VT *__restrict__ b, int K, int m, int C, int nch,
-                                                         VT *__restrict__ agg, int *flags, VT *x, int *status,
-                                                         long long limit) {
+                                                         const BT *__restrict__ b, long long rs, long long cs, int m,
+                                                         int C, int nch, VT *__restrict__ agg, int *flags, BT *x,
+                                                         int *status, long long limit) {
     extern __shared__ unsigned char smem_raw[];
     VT *sm = reinterpret_cast<VT *>(smem_raw);
     __shared__ VT s_state[W];
@@ -147,6 +155,8 @@ __global__ void __launch_bounds__(BAND_T) k_band_onepass(const VT *__restrict__ 
     const int tid = threadIdx.x, colk = blockIdx.y;
     const int nblk = band_blocks(nch);
     agg += (long long)colk * nblk * E;
+    b += (long long)colk * cs;
+    x += (long long)colk * cs;
     flags += (long long)colk * (nblk + 1);
     if (tid == 0) s_o = atomicAdd(flags, 1);  // this CTA's place in the chain
     __syncthreads();
@@ -168,7 +178,7 @@ __global__ void __launch_bounds__(BAND_T) k_band_onepass(const VT *__restrict__ 
         VT a[W];
 #pragma unroll
         for (int d = 0; d < W; ++d) a[d] = coef[oi * W + d];
-        band_step_M<VT, W>(M, c, a, inv[oi], b[(long long)(j * C + i) * K + colk]);
+        band_step_M<VT, W>(M, c, a, inv[oi], (VT)b[(long long)(j * C + i) * rs]);
     }
     band_cta_scan<VT, W>(M, c, sm);
 
@@ -206,25 +216,88 @@ __global__ void __launch_bounds__(BAND_T) k_band_onepass(const VT *__restrict__ 
                 if (it > 16) __nanosleep(64);
             }
         }
-        __syncthreads();
-        for (int i = tid; i < cnt * E; i += BAND_T) sm[i] = __ldcg(agg + (long long)base * E + i);
-        __syncthreads();
-        if (tid == 0) {
-            for (int q = 0; q < cnt; ++q) {
-                const VT *t = sm + (long long)q * E;
-                VT ns[W];
+        if constexpr (W <= 4) {
+            // the totals composed pairwise (thread t ends a run of 2 * off of
+            // them), so that hundreds of them cost eight rounds instead of a
+            // matrix-vector product each in a row (488 of them: 20 us)
+            VT Mt[W][W], ct[W];
+#pragma unroll
+            for (int r = 0; r < W; ++r) {
+#pragma unroll
+                for (int q = 0; q < W; ++q) Mt[r][q] = r == q ? VT(1) : VT(0);
+                ct[r] = 0;
+            }
+            if (tid < cnt) {
+                const VT *t = agg + (long long)(base + tid) * E;
 #pragma unroll
                 for (int r = 0; r < W; ++r) {
-                    VT v = t[W * W + r];
 #pragma unroll
-                    for (int k = 0; k < W; ++k) v += t[r * W + k] * s0[k];
-                    ns[r] = v;
+                    for (int q = 0; q < W; ++q) Mt[r][q] = __ldcg(t + r * W + q);
+                    ct[r] = __ldcg(t + W * W + r);
                 }
-#pragma unroll
-                for (int r = 0; r < W; ++r) s0[r] = ns[r];
             }
+            for (int off = 1; off < BAND_T; off <<= 1) {
+                if ((tid & (off - 1)) == off - 1) band_put<VT, W>(sm, BAND_T, tid, Mt, ct);
+                __syncthreads();
+                if ((tid & (2 * off - 1)) == 2 * off - 1) {
+                    VT Me[W][W], ce[W], nM[W][W], nc[W];
+                    band_get<VT, W>(sm, BAND_T, tid - off, Me, ce);
+#pragma unroll
+                    for (int r = 0; r < W; ++r) {
+                        VT v = ct[r];
+#pragma unroll
+                        for (int k = 0; k < W; ++k) v += Mt[r][k] * ce[k];
+                        nc[r] = v;
+#pragma unroll
+                        for (int q = 0; q < W; ++q) {
+                            VT u = 0;
+#pragma unroll
+                            for (int k = 0; k < W; ++k) u += Mt[r][k] * Me[k][q];
+                            nM[r][q] = u;
+                        }
+                    }
+#pragma unroll
+                    for (int r = 0; r < W; ++r) {
+                        ct[r] = nc[r];
+#pragma unroll
+                        for (int q = 0; q < W; ++q) Mt[r][q] = nM[r][q];
+                    }
+                }
+                __syncthreads();
+            }
+            if (tid == BAND_T - 1) {
+#pragma unroll
+                for (int r = 0; r < W; ++r) {
+                    VT v = ct[r];
+#pragma unroll
+                    for (int k = 0; k < W; ++k) v += Mt[r][k] * s0[k];
+                    s_state[r] = v;
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < W; ++r) s0[r] = s_state[r];
+        } else {
+            __syncthreads();
+            for (int i = tid; i < cnt * E; i += BAND_T) sm[i] = __ldcg(agg + (long long)base * E + i);
+            __syncthreads();
+            if (tid == 0) {
+                for (int q = 0; q < cnt; ++q) {
+                    const VT *t = sm + (long long)q * E;
+                    VT ns[W];
+#pragma unroll
+                    for (int r = 0; r < W; ++r) {
+                        VT v = t[W * W + r];
+#pragma unroll
+                        for (int k = 0; k < W; ++k) v += t[r * W + k] * s0[k];
+                        ns[r] = v;
+                    }
+#pragma unroll
+                    for (int r = 0; r < W; ++r) s0[r] = ns[r];
+                }
+            }
+            __syncthreads();
         }
-        __syncthreads();
     }
     if (tid == 0) {
 #pragma unroll
@@ -255,11 +328,11 @@ __global__ void __launch_bounds__(BAND_T) k_band_onepass(const VT *__restrict__ 
         VT acc = 0;
 #pragma unroll
         for (int d = 0; d < W; ++d) acc += coef[oi * W + d] * s[d];
-        const VT xp = inv[oi] * (b[(long long)p * K + colk] - acc);
+        const VT xp = inv[oi] * ((VT)b[(long long)p * rs] - acc);
 #pragma unroll
         for (int d = W - 1; d > 0; --d) s[d] = s[d - 1];
         s[0] = xp;
-        x[(long long)p * K + colk] = finalize(xp);
+        x[(long long)p * rs] = (BT)finalize(xp);
     }
 }
 

@@ -83,6 +83,11 @@ struct DeviceState {
     // strip layout of the whole matrix (level_strip.cuh); with it perm, ipos
     // and the full CSR are in strip order
     bool strip = false;
+    // band scan of the whole matrix (band.cuh); dir: rows are solved in the
+    // caller's order (1), its reverse (-1) or another (0)
+    bool band = false;
+    ExecBlock band_blk{};
+    int band_dir = 0;
     int strip_w = 0, strip_n = 0, strip_pub = 0;
     int *strip_first = nullptr, *strip_ticket = nullptr, *strip_rows = nullptr;
     unsigned char *strip_at = nullptr;
@@ -646,9 +651,10 @@ int syncfree_grid(const DeviceState &D) {
     return per_sm * D.num_sms;
 }
 
-// Band-scan triangle: three launches, each over all K right-hand sides (see band.cuh).
-template <typename VT, int W>
-int run_band(Plan &P, const ExecBlock &B, const VT *bb, VT *xx, int K, std::string &err) {
+// Band-scan triangle, or the whole matrix (see band.cuh): one launch over all
+// K right-hand sides; row p of column c at p * rs + c * cs of bb and xx.
+template <typename VT, int W, typename BT>
+int run_band(Plan &P, const ExecBlock &B, const BT *bb, BT *xx, long long rs, long long cs, int K, std::string &err) {
     DeviceState &D = *P.dev;
     cudaStream_t st = D.stream;
     const VT *coef = Pools<VT>::bcoef(D) + B.band_off;
@@ -659,7 +665,7 @@ int run_band(Plan &P, const ExecBlock &B, const VT *bb, VT *xx, int K, std::stri
     const size_t smem = (size_t)BAND_T * E * sizeof(VT);
     static std::atomic<unsigned long long> attr_set{0};
     if (!attr_done(attr_set)) {
-        CK(cudaFuncSetAttribute(k_band_onepass<VT, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(cudaFuncSetAttribute(k_band_onepass<VT, W, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_mark(attr_set);
     }
     const int nch = B.band_nch, nblk = band_blocks(nch);
@@ -667,9 +673,19 @@ int run_band(Plan &P, const ExecBlock &B, const VT *bb, VT *xx, int K, std::stri
     // and the CTAs' ready flags (nblk + 1 ints) in the states scratch
     int *flags = reinterpret_cast<int *>(states);
     CK(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)K * (nblk + 1), st));
-    k_band_onepass<VT, W><<<dim3(nblk, K), BAND_T, smem, st>>>(coef, binv, bb, K, B.m, B.band_c, nch, maps, flags, xx,
-                                                             D.status, P.opt.spin_limit);
+    k_band_onepass<VT, W, BT><<<dim3(nblk, K), BAND_T, smem, st>>>(coef, binv, bb, rs, cs, B.m, B.band_c, nch, maps, flags,
+                                                                xx, D.status, P.opt.spin_limit);
     return RBS_OK;
+}
+
+template <typename VT, typename BT>
+int run_band_any(Plan &P, const ExecBlock &B, const BT *bb, BT *xx, long long rs, long long cs, int K, std::string &err) {
+    switch (B.band_w) {
+    case 1: return run_band<VT, 1, BT>(P, B, bb, xx, rs, cs, K, err);
+    case 2: return run_band<VT, 2, BT>(P, B, bb, xx, rs, cs, K, err);
+    case 4: return run_band<VT, 4, BT>(P, B, bb, xx, rs, cs, K, err);
+    default: return run_band<VT, 8, BT>(P, B, bb, xx, rs, cs, K, err);
+    }
 }
 
 // Grouped-layout moves of the processing positions [pa, pb) on stream st
@@ -962,12 +978,13 @@ template <typename VT, int K>
 int launch_blocks(Plan &P, std::string &err, bool io = false) {
     DeviceState &D = *P.dev;
     cudaStream_t st = D.stream;
-    if (D.la || D.strip) {  // profiled walks report the whole launch as the first block's time
+    if (D.la || D.strip || D.band) {  // profiled walks report the whole launch as the first block's time
         for (const ExecBlock &B : P.blocks) {
             if (D.profile) CK(cudaEventRecord(D.bev[2 * B.index], st));
             if (B.index == 0) {
                 int rc = RBS_ERR_UNSUPPORTED;
-                if (D.la) rc = launch_la<VT>(P, K, err);
+                if (D.band) rc = run_band_any<VT, VT>(P, D.band_blk, Pools<VT>::bw(D), Pools<VT>::xw(D), K, 1, K, err);
+                else if (D.la) rc = launch_la<VT>(P, K, err);
                 else if constexpr (sizeof(VT) == 4) rc = launch_strip<VT>(P, K, err);  // FP64 walks run on the caller's vectors
                 if (rc) return rc;
             }
@@ -1131,13 +1148,7 @@ int launch_blocks(Plan &P, std::string &err, bool io = false) {
                 k_tri_seq<VT, K><<<1, 32, 0, st>>>(D.rp + B.rp_off, D.col, val, inv + B.r0, bb, xx, B.m);
                 break;
             case RBS_K_BANDSCAN: {
-                int rc2 = RBS_OK;
-                switch (B.band_w) {
-                case 1: rc2 = run_band<VT, 1>(P, B, bb, xx, K, err); break;
-                case 2: rc2 = run_band<VT, 2>(P, B, bb, xx, K, err); break;
-                case 4: rc2 = run_band<VT, 4>(P, B, bb, xx, K, err); break;
-                default: rc2 = run_band<VT, 8>(P, B, bb, xx, K, err); break;
-                }
+                const int rc2 = run_band_any<VT, VT>(P, B, bb, xx, K, 1, K, err);
                 if (rc2) return rc2;
                 break;
             }
@@ -1222,7 +1233,7 @@ int launch_blocks(Plan &P, std::string &err, bool io = false) {
 // vector for its sentinel (the sync-free kernels), with the kernel choice
 // of launch_blocks.
 bool walk_polls(const Plan &P, int K) {
-    if (P.dev->la || P.dev->strip) return false;
+    if (P.dev->la || P.dev->strip || P.dev->band) return false;
     for (const ExecBlock &B : P.blocks) {
         if (!B.tri) continue;
         if (B.kernel == RBS_K_SYNCFREE) return true;
@@ -1243,7 +1254,7 @@ int run_blocks(Plan &P, std::string &err, bool io = false) {
     }
     // per-block timing needs real event timestamps, which captured event
     // records are not: profiled solves launch eagerly
-    if (!D.use_graphs || D.profile || D.la || D.strip) return launch_blocks<VT, K>(P, err, io);
+    if (!D.use_graphs || D.profile || D.la || D.strip || D.band) return launch_blocks<VT, K>(P, err, io);
     const long long key = (long long)K * 8 + (sizeof(VT) == 8 ? 0 : 2) + (io ? 4 : 0);
     auto it = D.graphs.find(key);
     if (it != D.graphs.end()) {
@@ -1333,6 +1344,23 @@ void scatter_out(DeviceState &D, int n, VT *xw, int k, double *x, int ld, double
     }
 }
 
+// Whole-matrix band scan on the caller's columns.
+template <typename VT>
+int solve_band(Plan &P, const double *b, double *x, int k, int ld, std::string &err) {
+    DeviceState &D = *P.dev;
+    if (D.profile)
+        for (const ExecBlock &B : P.blocks) {
+            CK(cudaEventRecord(D.bev[2 * B.index], D.stream));
+            if (B.index) CK(cudaEventRecord(D.bev[2 * B.index + 1], D.stream));
+        }
+    const long long o = D.band_dir > 0 ? 0 : P.n - 1;
+    int rc = run_band_any<VT, double>(P, D.band_blk, b + o, x + o, D.band_dir, ld, k, err);
+    if (rc) return rc;
+    CK(cudaGetLastError());
+    if (D.profile) CK(cudaEventRecord(D.bev[1], D.stream));
+    return RBS_OK;
+}
+
 // Several columns in the grouped layout: the walk moves the columns itself,
 // overlapped with the blocks (launch_blocks), reading them through the device
 // table D.iotab set just before it on the same stream.
@@ -1340,6 +1368,7 @@ template <int K>
 int solve_fp64(Plan &P, const double *b, double *x, int k, int ld, std::string &err) {
     DeviceState &D = *P.dev;
     if (D.strip) return solve_strip<double>(P, b, x, nullptr, nullptr, k, ld, err);
+    if (D.band && D.band_dir) return solve_band<double>(P, b, x, k, ld, err);
     const int GL = plan_group<double>(P, K);
     if (K > 1 && GL && !D.la) {
         int rc = ensure_io_rows(P, err);
@@ -1362,6 +1391,7 @@ template <int K>
 int solve_fp32(Plan &P, const double *b, double *x, int k, int ld, std::string &err) {
     DeviceState &D = *P.dev;
     if (D.strip) return solve_strip<float>(P, b, x, nullptr, nullptr, k, ld, err);
+    if (D.band && D.band_dir) return solve_band<float>(P, b, x, k, ld, err);
     const int GL = plan_group<float>(P, K);
     if (K > 1 && GL && !D.la) {
         int rc = ensure_io_rows(P, err);
@@ -1713,6 +1743,81 @@ int upload_strips(Plan &P, std::string &err) {
     return RBS_OK;
 }
 
+// Band layout of the whole matrix, when the cost model gave every triangle
+// with off-diagonal entries to the band scan and no row reaches further than
+// 8 positions back across the triangles either (D.band stays false
+// otherwise).  Row r is row r % C of chunk r / C, as in a triangle's layout.
+int upload_band(Plan &P, std::string &err) {
+    DeviceState &D = *P.dev;
+    if (P.opt.select != RBS_SELECT_AUTO || P.blocks.size() < 2) return RBS_OK;
+    bool any = false;
+    for (const ExecBlock &B : P.blocks) {
+        if (!B.tri || B.nnz == B.m) continue;
+        if (B.kernel != RBS_K_BANDSCAN) return RBS_OK;
+        any = true;
+    }
+    if (!any) return RBS_OK;
+    const int n = P.n;
+    constexpr int kRows = 1 << 14;
+    std::atomic<int> reach{1};
+    parallel_for(((size_t)n + kRows - 1) / kRows, [&](size_t g) {
+        int top = 1;
+        for (int p = (int)g * kRows; p < std::min(n, (int)g * kRows + kRows); ++p)
+            for (int k = P.full_rp[(size_t)p]; k < P.full_rp[(size_t)p + 1]; ++k) top = std::max(top, p - P.full_col[(size_t)k]);
+        for (int old = reach.load(); top > old && !reach.compare_exchange_weak(old, top);) {
+        }
+    });
+    if (reach > 8) return RBS_OK;
+    ExecBlock &B = D.band_blk;
+    B = ExecBlock{};
+    B.tri = 1;
+    B.m = n;
+    int W = 1;
+    while (W < reach) W <<= 1;
+    B.band_w = W;
+    // rows per chunk: one CTA per SM, as every CTA's scans cost the same
+    // however few rows it has (1M rows: 8-row chunks 94, 16 rows
+    // 61, 32 rows 49 us)
+    B.band_c = std::max(4, W);
+    while (((long long)n + B.band_c - 1) / B.band_c > (long long)D.num_sms * BAND_T) B.band_c <<= 1;
+    B.band_nch = (n + B.band_c - 1) / B.band_c;
+    const size_t slots = (size_t)B.band_nch * B.band_c;
+    bulk_vector<double> coef(slots * W), inv(slots);
+    std::atomic<int> fwd{1}, bwd{1};
+    const int C = B.band_c, nch = B.band_nch;
+    parallel_for(((size_t)nch + 1023) / 1024, [&](size_t g) {
+        bool f = true, r = true;
+        // a chunk's rows lie nch slots apart
+        for (int i = 0; i < C; ++i)
+            for (int j = (int)g * 1024; j < std::min(nch, (int)g * 1024 + 1024); ++j) {
+                const size_t o = (size_t)i * nch + j;
+                double *a = coef.data() + o * W;
+                for (int d = 0; d < W; ++d) a[d] = 0.0;
+                inv[o] = 0.0;
+                const long long p = (long long)j * C + i;
+                if (p >= n) continue;
+                inv[o] = P.inv_diag[(size_t)p];
+                for (int k = P.full_rp[(size_t)p]; k < P.full_rp[(size_t)p + 1]; ++k)
+                    if (P.full_col[(size_t)k] != p) a[p - P.full_col[(size_t)k] - 1] += P.full_val[(size_t)k];
+                f = f && P.perm[(size_t)p] == p;
+                r = r && P.perm[(size_t)p] == n - 1 - p;
+            }
+        if (!f) fwd = 0;
+        if (!r) bwd = 0;
+    });
+    D.band_dir = fwd ? 1 : bwd ? -1 : 0;
+    int rc;
+    if ((rc = upload(D, D.band_coef, coef, err)) || (rc = upload(D, D.band_inv, inv, err))) return rc;
+    if (D.mixed) {
+        const auto c32 = to_f32(coef), i32 = to_f32(inv);
+        if ((rc = upload(D, D.band_coef32, c32, err)) || (rc = upload(D, D.band_inv32, i32, err))) return rc;
+    }
+    D.band_maps1 = (size_t)band_blocks(nch) * (W * W + W);
+    D.band_states1 = ((size_t)band_blocks(nch) + 1) * sizeof(int) / sizeof(double) + 1;
+    D.band = true;
+    return RBS_OK;
+}
+
 // The blocks' pools and per-kernel layouts (the block walk).
 int upload_blocks(Plan &P, std::string &err) {
     DeviceState &D = *P.dev;
@@ -1831,8 +1936,9 @@ int device_build(Plan &P, std::string &err) {
             if ((rc = upload(D, D.full_val, P.full_val, err))) return rc;
         }
         if (wants_la(P) && (rc = upload_la(P, err))) return rc;
+        if (!D.la && (rc = upload_band(P, err))) return rc;
     }
-    if (!D.la && !D.strip && (rc = upload_blocks(P, err))) return rc;
+    if (!D.la && !D.strip && !D.band && (rc = upload_blocks(P, err))) return rc;
     {
         int prio_low = 0, prio_high = 0;
         CK(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
