@@ -15,6 +15,14 @@
 // a row's updates happen in the serial order, so the factor is bit-identical
 // to the serial IKJ algorithm.
 //
+// Rows of at most 32 entries (k_ilu0_short): the row lives in the warp's
+// registers, a lane per entry, and each entry is written once, when it is
+// final, over a sentinel that arithmetic never produces -- so a dependency is
+// waited for and read by the same load, and the pattern matches against the
+// dependencies' rows are found before they are ready.  A level then costs one
+// trip through L2 and the division, instead of a flag, two dependent loads and
+// a search per dependency (2D 5-point matrix, 1M rows: kernel 14.4 -> 3.1 ms).
+//
 // IC(0) (incomplete Cholesky, zero fill) of an SPD matrix given as its lower
 // triangle uses the same scheme: row i computes l_ik = (a_ik - sum_{j<k}
 // l_ij l_kj) / l_kk for its columns k in ascending order, the products over
@@ -24,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -35,6 +44,7 @@ namespace rbs {
 
 namespace {
 
+constexpr int ILU_SHORT = 32;  // entries of a row kept in a warp's registers
 constexpr int ILU_MISSING_DIAG = 2, ILU_UNSORTED = 4, ILU_ZERO_PIVOT = 8, IC_NOT_LOWER = 16, IC_NOT_POSITIVE = 32;
 constexpr unsigned FULL = 0xffffffffu;
 
@@ -50,7 +60,8 @@ __device__ __forceinline__ void st_release_int(int *p, int v) {
 // diagonal position of every row; the row pointer must be valid and the
 // columns in range and ascending (checked before any of them is used)
 __global__ void k_ilu0_diag(const int *__restrict__ rp, const int *__restrict__ ci, int n, int nnz, int *diag,
-                            int *status, int *bad_row) {
+                            int *status, int *bad_row, int *longest) {
+    int most = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int d = -1, flag = 0;
         const int b = rp[i], e = rp[i + 1];
@@ -62,8 +73,84 @@ __global__ void k_ilu0_diag(const int *__restrict__ rp, const int *__restrict__ 
             }
         if (d < 0) flag |= ILU_MISSING_DIAG;
         diag[i] = d;
+        most = max(most, e - b);
         if (flag) {
             atomicOr(status, flag);
+            atomicMin(bad_row, i);
+        }
+    }
+    most = __reduce_max_sync(FULL, most);
+    if ((threadIdx.x & 31) == 0) atomicMax(longest, most);
+}
+
+// Rows of at most 32 entries; lu is filled with the sentinel before.
+__global__ void __launch_bounds__(128) k_ilu0_short(const int *__restrict__ rp, const int *__restrict__ ci,
+                                                    const int *__restrict__ diag, const int *__restrict__ order,
+                                                    const double *__restrict__ val, double *lu, int n, int *ticket,
+                                                    int *status, int *bad_row, long long limit) {
+    constexpr int D = 4;  // dependencies whose matches are found ahead
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(ticket, 1);
+        t = __shfl_sync(FULL, t, 0);
+        if (t >= n) return;
+        const int i = order[t];
+        const int s = rp[i], len = rp[i + 1] - s, nd = diag[i] - s;
+        const int j = lane < len ? ci[s + lane] : -1;
+        double a = lane < len ? val[s + lane] : 0.0;
+        // lane p < nd: the pivot's place and the end of dependency p's row
+        int kd = 0, ke = 0;
+        if (lane < nd) {
+            kd = diag[j];
+            ke = rp[j + 1];
+        }
+        // place of the entry of dependency p's upper part in this lane's column, -1: none
+        auto match = [&](int p, int d) {
+            const int cnt = __shfl_sync(FULL, ke, p) - d - 1;
+            const int c = lane < cnt ? ci[d + 1 + lane] : -1;
+            int m = -1;
+            for (int u = 0; u < cnt; ++u)
+                if (__shfl_sync(FULL, c, u) == j) m = d + 1 + u;
+            return lane > p ? m : -1;
+        };
+        auto apply = [&](int p, double piv, double v, int m) {
+            const double l = __ddiv_rn(__shfl_sync(FULL, a, p), piv);
+            if (lane == p) a = l;
+            if (m >= 0) a = __dsub_rn(a, __dmul_rn(l, v));
+        };
+        int d[D], m[D];
+        double piv[D], v[D];
+#pragma unroll
+        for (int p = 0; p < D; ++p)
+            if (p < nd) {
+                d[p] = __shfl_sync(FULL, kd, p);
+                m[p] = match(p, d[p]);
+            }
+#pragma unroll
+        for (int p = 0; p < D; ++p)
+            if (p < nd) {  // all first loads together; what is not ready is polled below
+                piv[p] = ld_relaxed(lu + d[p]);
+                v[p] = m[p] >= 0 ? ld_relaxed(lu + m[p]) : 0.0;
+            }
+#pragma unroll
+        for (int p = 0; p < D; ++p)
+            if (p < nd) {
+                if (Sent<double>::is(piv[p])) piv[p] = wait_value(lu + d[p], status, limit);
+                if (Sent<double>::is(v[p])) v[p] = wait_value(lu + m[p], status, limit);
+                __syncwarp();
+                apply(p, piv[p], v[p], m[p]);
+            }
+        for (int p = D; p < nd; ++p) {
+            const int dp = __shfl_sync(FULL, kd, p), mp = match(p, dp);
+            const double pv = wait_value(lu + dp, status, limit);
+            const double vv = mp >= 0 ? wait_value(lu + mp, status, limit) : 0.0;
+            __syncwarp();
+            apply(p, pv, vv, mp);
+        }
+        if (lane < len) st_relaxed(lu + s + lane, finalize(a));
+        if (lane == nd && a == 0.0) {
+            atomicOr(status, ILU_ZERO_PIVOT);
             atomicMin(bad_row, i);
         }
     }
@@ -243,7 +330,7 @@ static int device_factor(bool ic, const int *d_rp, const int *d_ci, const double
         return RBS_ERR_CUDA;
     cudaStream_t st = nullptr;
     cudaMemPool_t pool = nullptr;  // the per-device stream-ordered pool (allocations on st)
-    int *scratch = nullptr;  // diag[n], done[n], ticket, status, bad_row
+    int *scratch = nullptr;  // diag[n], done[n], ticket, status, bad_row, longest row
     int rc = RBS_OK;
     if (!ck(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream") ||
         !ck(device_mem_pool(dev, pool), "memory pool") ||
@@ -252,16 +339,15 @@ static int device_factor(bool ic, const int *d_rp, const int *d_ci, const double
         rc = RBS_ERR_CUDA;
     int *diag = scratch, *done = scratch + n, *ticket = scratch + 2 * (size_t)n, *status = ticket + 1,
         *bad = ticket + 2;
-    int h[3] = {0, 0, 0};
+    int h[4] = {0, 0, 0, 0};
+    bool short_rows = false;
     if (rc == RBS_OK) {
-        const int bad0[3] = {0, 0, 0x7fffffff};
-        bool ok = ck(cudaMemsetAsync(done, 0, sizeof(int) * (size_t)n, st), "memset") &&
-                  ck(cudaMemcpyAsync(ticket, bad0, sizeof(bad0), cudaMemcpyHostToDevice, st), "memcpy") &&
-                  ck(cudaMemcpyAsync(d_lu, d_val, sizeof(double) * (size_t)nnz, cudaMemcpyDeviceToDevice, st), "memcpy");
+        const int bad0[4] = {0, 0, 0x7fffffff, 0};
+        bool ok = ck(cudaMemcpyAsync(ticket, bad0, sizeof(bad0), cudaMemcpyHostToDevice, st), "memcpy");
         if (ok) {
             const int g = (n + 255) / 256 < sms * 8 ? (n + 255) / 256 : sms * 8;
             if (ic) k_ic0_check<<<g, 256, 0, st>>>(d_rp, d_ci, n, nnz, diag, status, bad);
-            else k_ilu0_diag<<<g, 256, 0, st>>>(d_rp, d_ci, n, nnz, diag, status, bad);
+            else k_ilu0_diag<<<g, 256, 0, st>>>(d_rp, d_ci, n, nnz, diag, status, bad, ticket + 3);
             ok = ck(cudaGetLastError(), "launch") &&
                  ck(cudaMemcpyAsync(h, ticket, sizeof(h), cudaMemcpyDeviceToHost, st), "memcpy") &&
                  ck(cudaStreamSynchronize(st), "sync");
@@ -275,6 +361,23 @@ static int device_factor(bool ic, const int *d_rp, const int *d_ci, const double
                                            : " has no diagonal");
             rc = RBS_ERR_STRUCTURE;
         }
+    }
+    if (rc == RBS_OK) {
+        // a factor that overlaps the matrix's own values is computed in place
+        const double *v1 = d_val + nnz, *l1 = d_lu + nnz;
+        short_rows = !ic && h[3] <= ILU_SHORT && (l1 <= d_val || v1 <= d_lu);
+        bool ok = true;
+        if (short_rows) {
+            const unsigned long long bits = RBS_SENT64;
+            double sent;
+            std::memcpy(&sent, &bits, 8);
+            k_fill<double><<<sms * 16, 256, 0, st>>>(d_lu, (long long)nnz, sent);
+            ok = ck(cudaGetLastError(), "launch");
+        } else {
+            ok = ck(cudaMemsetAsync(done, 0, sizeof(int) * (size_t)n, st), "memset") &&
+                 ck(cudaMemcpyAsync(d_lu, d_val, sizeof(double) * (size_t)nnz, cudaMemcpyDeviceToDevice, st), "memcpy");
+        }
+        if (!ok) rc = RBS_ERR_CUDA;
     }
     // rows in dependency-level order (level of row i = 1 + the largest level
     // of the rows of its lower part; all of them precede i), ascending inside
@@ -306,6 +409,8 @@ static int device_factor(bool ic, const int *d_rp, const int *d_ci, const double
     }
     if (rc == RBS_OK) {
         if (ic) k_ic0<<<sms * 4, 256, 0, st>>>(d_rp, d_ci, order, d_lu, n, ticket, done, status, bad, opt.spin_limit);
+        else if (short_rows)
+            k_ilu0_short<<<sms * 12, 128, 0, st>>>(d_rp, d_ci, diag, order, d_val, d_lu, n, ticket, status, bad, opt.spin_limit);
         else k_ilu0<<<sms * 4, 256, 0, st>>>(d_rp, d_ci, diag, order, d_lu, n, ticket, done, status, bad, opt.spin_limit);
         if (!ck(cudaGetLastError(), "launch") ||
             !ck(cudaMemcpyAsync(h, ticket, sizeof(h), cudaMemcpyDeviceToHost, st), "memcpy") ||
