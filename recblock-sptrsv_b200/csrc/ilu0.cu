@@ -7,8 +7,8 @@
 // the row (ascending), a_ik /= a_kk, then a_ij -= a_ik * a_kj for every j > k
 // present in both rows i and k.  Row i needs rows k < i of its lower part to
 // be final, so one warp takes one row at a time in ticket order -- rows
-// sorted by dependency level (computed on the host from a copy of the
-// pattern), so the rows in flight span whole levels; the earliest
+// sorted by dependency level (k_row_levels, then a stable sort), so the rows
+// in flight span whole levels; the earliest
 // unfinished row always has a warp: no deadlock whatever the grid -- and
 // waits, bounded, on each dependency's completion flag (release/acquire).
 // Every product and difference is rounded separately (no contraction), and
@@ -29,12 +29,12 @@
 // the columns it shares with row k found by the lanes (binary search) and
 // subtracted in ascending column order through warp shuffles, then
 // l_ii = sqrt(a_ii - sum_j l_ij^2) -- the serial row algorithm bit for bit.
+#include <cub/cub.cuh>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
 #include <string>
-#include <vector>
 
 #include "kernels.cuh"
 #include "rbs.h"
@@ -81,6 +81,59 @@ __global__ void k_ilu0_diag(const int *__restrict__ rp, const int *__restrict__ 
     }
     most = __reduce_max_sync(FULL, most);
     if ((threadIdx.x & 31) == 0) atomicMax(longest, most);
+}
+
+// Dependency level of every row (1 + the largest among the rows of its lower
+// part): a warp takes 32 consecutive rows, a lane each; dependencies outside
+// them are polled (level starts at -1), those inside resolved in lane order.
+// The host's walk over a copy of the pattern took about 10 ms of the 1M-row
+// matrix's call, with the copies; this takes 1.5 ms.
+__global__ void __launch_bounds__(256) k_row_levels(const int *__restrict__ rp, const int *__restrict__ ci, int n, int *level,
+                                                    int *rows, int *ticket, int *status, int *deepest, long long limit) {
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        int base = 0;
+        if (lane == 0) base = atomicAdd(ticket, 32);
+        base = __shfl_sync(FULL, base, 0);
+        if (base >= n) return;
+        const int i = base + lane;
+        int lv = 0;
+        unsigned inside = 0;  // this row's dependencies among the warp's rows
+        if (i < n) {
+            const int e = rp[i + 1];
+            for (int p = rp[i]; p < e; ++p) {
+                const int k = ci[p];
+                if (k >= i) break;
+                if (k >= base) {
+                    inside |= 1u << (k - base);
+                    continue;
+                }
+                int l;
+                for (long long it = 0;; ++it) {
+                    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(l) : "l"(level + k) : "memory");
+                    if (l >= 0) break;
+                    if (it >= limit) {
+                        atomicOr(status, RBS_STATUS_TIMEOUT);
+                        l = 0;
+                        break;
+                    }
+                    if (it > 64) __nanosleep(32);
+                }
+                lv = max(lv, l + 1);
+            }
+        }
+        __syncwarp();
+        for (int u = 0; u < 31; ++u) {
+            const int l = __shfl_sync(FULL, lv, u);
+            if (inside >> u & 1) lv = max(lv, l + 1);
+        }
+        if (i < n) {
+            asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(level + i), "r"(lv) : "memory");
+            rows[i] = i;
+        }
+        const int top = __reduce_max_sync(FULL, lv);
+        if (lane == 0) atomicMax(deepest, top);
+    }
 }
 
 // Rows of at most 32 entries; lu is filled with the sentinel before.
@@ -383,27 +436,33 @@ static int device_factor(bool ic, const int *d_rp, const int *d_ci, const double
     // of the rows of its lower part; all of them precede i), ascending inside
     // a level: the rows in flight at a time span whole levels, and every
     // dependency of a row has an earlier ticket
-    int *order = nullptr;
+    int *order = nullptr, *lv = nullptr;  // order[n]; levels, sorted levels, rows, ticket, deepest
+    void *tmp = nullptr;
     if (rc == RBS_OK) {
-        std::vector<int> hrp((size_t)n + 1), hci((size_t)nnz), lvl((size_t)n, 0), ord((size_t)n);
-        bool ok = ck(cudaMemcpyAsync(hrp.data(), d_rp, sizeof(int) * ((size_t)n + 1), cudaMemcpyDeviceToHost, st), "memcpy") &&
-                  ck(cudaMemcpyAsync(hci.data(), d_ci, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToHost, st), "memcpy") &&
-                  ck(cudaStreamSynchronize(st), "sync");
+        const size_t N = (size_t)n;
+        bool ok = ck(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&order), sizeof(int) * N, pool, st),
+                     "cudaMallocFromPoolAsync") &&
+                  ck(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&lv), sizeof(int) * (3 * N + 2), pool, st),
+                     "cudaMallocFromPoolAsync") &&
+                  ck(cudaMemsetAsync(lv, 0xff, sizeof(int) * N, st), "memset") &&
+                  ck(cudaMemsetAsync(lv + 3 * N, 0, 2 * sizeof(int), st), "memset");
+        int *rows = ok ? lv + 2 * N : nullptr, top = 0;
         if (ok) {
-            int nlev = 0;
-            for (int i = 0; i < n; ++i) {
-                int l = 0;
-                for (int p = hrp[(size_t)i]; p < hrp[(size_t)i + 1] && hci[(size_t)p] < i; ++p) l = std::max(l, lvl[(size_t)hci[(size_t)p]] + 1);
-                lvl[(size_t)i] = l;
-                nlev = std::max(nlev, l + 1);
-            }
-            std::vector<int> start((size_t)nlev + 1, 0);
-            for (int i = 0; i < n; ++i) start[(size_t)lvl[(size_t)i] + 1]++;
-            for (int l = 0; l < nlev; ++l) start[(size_t)l + 1] += start[(size_t)l];
-            for (int i = 0; i < n; ++i) ord[(size_t)start[(size_t)lvl[(size_t)i]]++] = i;
-            ok = ck(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&order), sizeof(int) * (size_t)n, pool, st),
-                    "cudaMallocFromPoolAsync") &&
-                 ck(cudaMemcpyAsync(order, ord.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, st), "memcpy");
+            // 32 rows a warp; more warps than fit only queue
+            const long long ctas = ((long long)n + 255) / 256;
+            k_row_levels<<<(unsigned)(ctas < sms * 8 ? ctas : sms * 8), 256, 0, st>>>(d_rp, d_ci, n, lv, rows, lv + 3 * N, status,
+                                                                                lv + 3 * N + 1, opt.spin_limit);
+            ok = ck(cudaGetLastError(), "launch") &&
+                 ck(cudaMemcpyAsync(&top, lv + 3 * N + 1, sizeof(int), cudaMemcpyDeviceToHost, st), "memcpy") &&
+                 ck(cudaStreamSynchronize(st), "sync");
+        }
+        if (ok) {
+            int bits = 1;
+            while (bits < 31 && (top >> bits)) ++bits;
+            size_t bytes = 0;
+            ok = ck(cub::DeviceRadixSort::SortPairs(nullptr, bytes, lv, lv + N, rows, order, n, 0, bits, st), "sort") &&
+                 ck(cudaMallocFromPoolAsync(&tmp, bytes ? bytes : 1, pool, st), "cudaMallocFromPoolAsync") &&
+                 ck(cub::DeviceRadixSort::SortPairs(tmp, bytes, lv, lv + N, rows, order, n, 0, bits, st), "sort");
         }
         if (!ok) rc = RBS_ERR_CUDA;
     }
@@ -429,6 +488,8 @@ static int device_factor(bool ic, const int *d_rp, const int *d_ci, const double
         }
     }
     if (order) cudaFreeAsync(order, st);
+    if (lv) cudaFreeAsync(lv, st);
+    if (tmp) cudaFreeAsync(tmp, st);
     if (scratch) cudaFreeAsync(scratch, st);
     if (st) {
         cudaStreamSynchronize(st);
