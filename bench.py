@@ -13,9 +13,10 @@ write) before every timed solve: the factor (58.7 MB) fits in the 126 MB L2.
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
   python bench.py --side analysis|batched|blocks|ic0|ilu0|mtx|serve [--case c1b]
 
-The headline value is timed on the block walk replayed from its CUDA graph;
-the roofline's per-kernel times come from a second pass of the same steps
-with CUDA events around every block.  Side measurements (multi-RHS, other
+The headline value is timed on the plan's own walk (for this factor one
+launch of the strip kernel; plans of several kernels replay their block walk
+from a CUDA graph); the roofline's per-kernel times come from a second pass of
+the same steps with CUDA events around the walk's kernels.  Side measurements (multi-RHS, other
 structures, mixed precision, analysis, factors, Matrix Market input,
 batched systems, serving) follow on one GPU; --side runs one alone.
 
@@ -839,7 +840,8 @@ def side_serving(dev, args, n_requests=1000, loads=(500, 1000, 2000, 10000, 5000
 def profiled_traffic(kind):
     """DRAM bytes (read + write) per launch of the dominant kernel from the
     committed ncu summary of the same workload (profiles/), or None."""
-    path = {"level": os.path.join(ROOT, "profiles", "k_tri_level_ca_c1a.md")}.get(kind)
+    path = {"level": os.path.join(ROOT, "profiles", "k_tri_level_ca_c1a.md"),
+            "k_tri_strip": os.path.join(ROOT, "profiles", "k_tri_strip_c1a.md")}.get(kind)
     if not path or not os.path.exists(path):
         return None
     for line in open(path):
@@ -850,6 +852,9 @@ def profiled_traffic(kind):
 
 def launches_per_solve(plan):
     import rbs
+    walk, launches = plan.export("walk")
+    if walk:  # a whole-matrix walk
+        return int(launches)
     kern = plan.export("kernel")
     lr = plan.export("longrow")
     mr = plan.export("medrow")
@@ -922,17 +927,23 @@ def run_ours(args):
     dom_ms_per_solve = by_kind[dom][0] / max(solves, 1)
     dom_launch_ms = dom_ms_per_solve / by_kind[dom][2]
     dom_bytes_per_launch = by_kind[dom][1] / by_kind[dom][2]
+    dom_name = rbs.KERNEL_NAMES[dom]
+    walk = int(plan.export("walk")[0])
+    if walk:  # one launch walks the whole matrix; it is timed as the first block
+        dom_name = ["", "k_tri_la", "k_tri_strip", "k_band_onepass"][walk]
+        dom_launch_ms = sum(v[0] for v in by_kind.values()) / max(solves, 1)
+        dom_bytes_per_launch = useful
     peak, peak_kind = peaks()
     achieved = dom_bytes_per_launch / (dom_launch_ms / 1000) / 1e9
-    traffic = profiled_traffic(rbs.KERNEL_NAMES[dom])
+    traffic = profiled_traffic(dom_name)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic, "peak_source": peak_kind, "kernel": rbs.KERNEL_NAMES[dom],
-                "kernel_share": by_kind[dom][0] / max(sum(v[0] for v in by_kind.values()), 1e-30),
+                "traffic": traffic, "peak_source": peak_kind, "kernel": dom_name,
+                "kernel_share": 1.0 if walk else by_kind[dom][0] / max(sum(v[0] for v in by_kind.values()), 1e-30),
                 "bytes_per_launch": dom_bytes_per_launch, "launch_ms": dom_launch_ms,
                 "solve_frac": useful / (ms_per_step / 1000) / 1e9 / peak,
                 "timing": "per-block CUDA events on the plan's stream, second pass of the same steps "
                           f"(eager launches: {float(np.mean(pms)):.3f} ms per solve against "
-                          f"{ms_per_step:.3f} ms replayed from the graph)"}
+                          f"{ms_per_step:.3f} ms without them)"}
     plan.profile(False)
 
     if args.no_extras:

@@ -122,10 +122,23 @@ int pick_group(double avg) {
 // Kernel choice.  REFERENCE maps each reference method to this library's
 // kernel of the same kind; AUTO uses a latency/bandwidth cost model of the
 // B200 (constants measured on a B200 with bench.py).
-// nseg: independent systems of a batch (1 otherwise).  The single-CTA level
-// kernels run them side by side, one per CTA, so their time is the longest
-// system's levels or an even share of the bytes.
-void select_kernel(ExecBlock &b, const rbs_options &opt, const std::vector<int> &lvl_sizes, int nseg) {
+// Whether a single-CTA level kernel is the better choice for a triangle once
+// its levels may run on the look-ahead kernel (the whole-matrix walk; the
+// block walk keeps select_kernel's choice).  nseg: independent systems of a
+// batch (1 otherwise), which run side by side, one per CTA, so their time is
+// the longest system's levels or an even share of the bytes.  The one-warp
+// kernel takes 0.69 us a row (8,000 rows with 1,298 levels: 5.6 ms, against 0.3
+// us a level), which select_kernel puts far lower.
+bool level_preferred(const ExecBlock &b, const std::vector<int> &lvl_sizes, int nseg) {
+    if (b.kernel != RBS_K_SEQ && b.kernel != RBS_K_SYNCFREE) return b.kernel == RBS_K_LEVEL;
+    const double off = b.nnz - b.m, bytes = off * 12.0 + (double)b.m * 24.0;
+    const double ctas = std::max(1, std::min(nseg, 148));
+    double passes = 0;
+    for (int w : lvl_sizes) passes += std::max(1.0, std::ceil((double)w * b.group / (1024.0 * ctas)));
+    return passes * 0.12 + bytes / (180e3 * ctas) + 4.0 < (double)b.nlv * 0.9 + bytes / 4.0e6 + 4.0;
+}
+
+void select_kernel(ExecBlock &b, const rbs_options &opt, const std::vector<int> &lvl_sizes) {
     if (!b.tri) {
         if (b.nnz == 0) {
             b.kernel = RBS_K_EMPTY;
@@ -158,14 +171,11 @@ void select_kernel(ExecBlock &b, const rbs_options &opt, const std::vector<int> 
     }
     // AUTO cost model (microseconds).
     double bytes = (double)off * 12.0 + (double)b.m * 24.0;
-    const double ctas = std::max(1, std::min(nseg, 148));
     double passes = 0;
-    for (int w : lvl_sizes) passes += std::max(1.0, std::ceil((double)w * b.group / (1024.0 * ctas)));
-    double t_level = passes * 0.12 + bytes / (180e3 * ctas) + 4.0;
+    for (int w : lvl_sizes) passes += std::max(1.0, std::ceil((double)w * b.group / 1024.0));
+    double t_level = passes * 0.12 + bytes / 180e3 + 4.0;
     double t_sync = (double)b.nlv * 0.9 + bytes / 4.0e6 + 4.0;
-    // one warp, one row after another: 0.69 us a row measured (8,000 rows with
-    // 1,298 levels: 5.6 ms, against 0.3 us a level in the level kernels)
-    double t_seq = (double)b.m * 0.69 + bytes / 120e3 + 4.0;
+    double t_seq = (double)b.m * 0.012 + bytes / 120e3 + 4.0;
     double t_scan = b.bandwidth <= 8 ? bytes * 3.0 / 3.0e6 + 25.0 : 1e30;
     double best = t_sync;
     b.kernel = RBS_K_SYNCFREE;
@@ -627,15 +637,44 @@ static void build_lc(Plan &P, const rbs_options &opt, const std::vector<int> &le
     P.lc_segs.swap(all.segs);
 }
 
-// The cost model chose a single-CTA level kernel for every triangle that has
-// off-diagonal entries, and at least one of them has rows or levels beyond
-// the staged level-ELL kernel's.
-bool wants_la(const Plan &P) {
+// Local level of every row from the triangles' entries: a recurrence in row
+// order.
+static std::vector<int> local_levels(const Plan &P) {
+    std::vector<int> level((size_t)P.n, 0);
+    parallel_for(P.blocks.size(), [&](size_t b) {
+        const ExecBlock &B = P.blocks[b];
+        if (!B.tri) return;
+        const int *rp = P.rp_pool.data() + B.rp_off;
+        int *lv = level.data() + B.r0;
+        for (int r = 0; r < B.m; ++r) {
+            int top = -1;
+            for (int k = rp[r]; k < rp[r + 1]; ++k) top = std::max(top, lv[P.col_pool[(size_t)k]]);
+            lv[r] = top + 1;
+        }
+    });
+    return level;
+}
+
+// A single-CTA level kernel is the better choice for every triangle that has
+// off-diagonal entries (level_preferred), and at least one of them has rows
+// or levels beyond the staged level-ELL kernel's.
+bool wants_la(Plan &P) {
     if (P.opt.select != RBS_SELECT_AUTO) return false;
+    if (P.level_better.size() != P.blocks.size()) {  // a loaded plan
+        const std::vector<int> level = local_levels(P);
+        P.level_better.assign(P.blocks.size(), 0);
+        for (size_t b = 0; b < P.blocks.size(); ++b) {
+            const ExecBlock &B = P.blocks[b];
+            if (!B.tri) continue;
+            std::vector<int> sizes((size_t)B.nlv, 0);
+            for (int r = 0; r < B.m && B.nnz > B.m; ++r) ++sizes[(size_t)level[(size_t)B.r0 + r]];
+            P.level_better[b] = level_preferred(B, sizes, std::max(1, (int)P.seg_rows.size()));
+        }
+    }
     bool any = false;
     for (const ExecBlock &B : P.blocks) {
         if (!B.tri || B.nnz == B.m) continue;
-        if (B.kernel != RBS_K_LEVEL) return false;
+        if (!P.level_better[(size_t)(&B - P.blocks.data())]) return false;
         any = any || !B.ca_ok;
     }
     return any;
@@ -658,20 +697,7 @@ bool wants_strips(const Plan &P) {
 void ensure_lc(Plan &P) {
     if (!P.lc_deferred) return;
     P.lc_deferred = false;
-    // local levels from the triangles' entries: a recurrence in row order
-    std::vector<int> level((size_t)P.n, 0);
-    parallel_for(P.blocks.size(), [&](size_t b) {
-        const ExecBlock &B = P.blocks[b];
-        if (!B.tri) return;
-        const int *rp = P.rp_pool.data() + B.rp_off;
-        int *lv = level.data() + B.r0;
-        for (int r = 0; r < B.m; ++r) {
-            int top = -1;
-            for (int k = rp[r]; k < rp[r + 1]; ++k) top = std::max(top, lv[P.col_pool[(size_t)k]]);
-            lv[r] = top + 1;
-        }
-    });
-    build_lc(P, P.opt, level);
+    build_lc(P, P.opt, local_levels(P));
 }
 
 int host_bfs_levels(const int *cp, const int *ri, int m, std::vector<int> &levelPtr, std::vector<int> &item) {
@@ -955,6 +981,7 @@ int analyse_after_levels(Plan &P, int n, int nnz, int substitution, int lv, cons
     // block statistics, the reference's method codes and the kernel choice:
     // blocks are independent, done on host threads
     std::vector<std::vector<int>> lvl_sizes((size_t)P.sum_block);
+    P.level_better.assign((size_t)P.sum_block, 0);
     parallel_for((size_t)P.sum_block, [&](size_t bi) {
         const int b = (int)bi;
         ExecBlock &B = P.blocks[b];
@@ -1011,7 +1038,8 @@ int analyse_after_levels(Plan &P, int n, int nnz, int substitution, int lv, cons
                 else B.ref_method = 3;
             }
         }
-        select_kernel(B, opt, lvl_sizes[b], std::max(1, (int)P.seg_rows.size()));
+        select_kernel(B, opt, lvl_sizes[b]);
+        if (B.tri) P.level_better[bi] = level_preferred(B, lvl_sizes[b], std::max(1, (int)P.seg_rows.size()));
         // The sync-free kernel's lane group.  A deep triangle (32 levels or
         // more) is bound by its level chain, where each level waits for its
         // longest rows: there the group is sized for the rows' tail, the

@@ -310,7 +310,14 @@ int rbs_plan_export(const rbs_plan *plan, const char *name, void *dst, long long
     std::string err;
     int rc;
     try {
-        rc = rbs::export_reference(plan->p, name, iv, dv, is_double, err);
+        // which walk a solve takes (0 blocks, 1 look-ahead, 2 strips, 3 whole band
+        // scan) and its kernel launches for one FP64 column (blocks: 0)
+        if (std::string(name) == "walk") {
+            rbs::device_walk(plan->p, iv);
+            rc = RBS_OK;
+        } else {
+            rc = rbs::export_reference(plan->p, name, iv, dv, is_double, err);
+        }
     } catch (const std::bad_alloc &) {
         return fail(RBS_ERR_NOMEM, "rbs_plan_export: out of host memory");
     }

@@ -266,6 +266,7 @@ struct Plan {
     // out until they are asked for (ensure_lc); the look-ahead layout is kept
     // here from the analysis to the upload.
     bool lc_deferred = false;
+    std::vector<char> level_better;  // per block, level_preferred (not saved)
     std::shared_ptr<LaHost> la;
     std::shared_ptr<StripHost> strip;  // the same for the strip kernel
     // original-row offsets of independent systems (batched plans); empty
@@ -335,7 +336,7 @@ int analyse_after_levels(Plan &P, int n, int nnz, int substitution, int lv, cons
                          const std::vector<int> *seg_rows = nullptr, DevRows *dev_rows = nullptr);
 
 // analysis.cpp: whether the plan's whole walk is the look-ahead kernel's work
-bool wants_la(const Plan &P);
+bool wants_la(Plan &P);
 // analysis.cpp: builds the level-chunk records a plan left out
 void ensure_lc(Plan &P);
 // analysis.cpp: whether strips are worth trying for the plan's whole walk
@@ -423,6 +424,8 @@ int device_batch_next(Plan &P, int *more, std::string &err);
 int device_batch_finish(Plan &P, int *iters, double *corr, std::string &err);
 double block_bytes(const Plan &P, const ExecBlock &B);
 long long device_bytes(const Plan &P);
+// the walk a solve takes and its kernel launches for one FP64 column
+void device_walk(const Plan &P, std::vector<int> &out);
 
 void set_error(const std::string &msg);
 

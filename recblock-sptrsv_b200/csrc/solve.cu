@@ -100,6 +100,11 @@ struct DeviceState {
     Exchange<double> ex64;
     Exchange<float> ex32;
     uint32_t *strip_rec64 = nullptr, *strip_rec32 = nullptr;
+    // the block walk's state beside a whole-matrix walk's: FP32 solves keep it,
+    // whose rounding depends on the order of every sum; built on the first one
+    DeviceState *shadow = nullptr;
+    bool bat_shadow = false;  // the batch in flight runs there
+    bool whole() const { return la || strip || band; }
     int wn = 0;  // positions of the work vectors (rows, or more with padding)
     int *la_queue = nullptr;  // one segment counter per column
     cudaStream_t side = nullptr;                         // L2 prefetch stream; moves of the overlapped walk
@@ -1390,8 +1395,6 @@ int solve_fp64(Plan &P, const double *b, double *x, int k, int ld, std::string &
 template <int K>
 int solve_fp32(Plan &P, const double *b, double *x, int k, int ld, std::string &err) {
     DeviceState &D = *P.dev;
-    if (D.strip) return solve_strip<float>(P, b, x, nullptr, nullptr, k, ld, err);
-    if (D.band && D.band_dir) return solve_band<float>(P, b, x, k, ld, err);
     const int GL = plan_group<float>(P, K);
     if (K > 1 && GL && !D.la) {
         int rc = ensure_io_rows(P, err);
@@ -1527,9 +1530,7 @@ int batch_start_k(Plan &P, const double *const *bcols, double *const *xcols, int
     DeviceState &D = *P.dev;
     const int n = P.n;
     int rc;
-    if (D.strip && prec != RBS_PREC_MIXED)
-        return prec == RBS_PREC_FP64 ? solve_strip<double>(P, nullptr, nullptr, bcols, xcols, k, n, err)
-                                     : solve_strip<float>(P, nullptr, nullptr, bcols, xcols, k, n, err);
+    if (D.strip && prec == RBS_PREC_FP64) return solve_strip<double>(P, nullptr, nullptr, bcols, xcols, k, n, err);
     if (prec == RBS_PREC_FP64) {
         const int GL = plan_group<double>(P, K);
         gather_in<double, double, K>(D, n, nullptr, n, bcols, k, D.bw64, nullptr, GL, gb);
@@ -1574,8 +1575,17 @@ int device_reserve(Plan &P, int k, std::string &err) {
     return RBS_OK;
 }
 
+template <typename F> static int on_shadow(Plan &P, std::string &err, F &&f);
+
 int device_batch_start(Plan &P, const double *const *bcols, double *const *xcols, int k, int prec, int *more,
                        std::string &err, const BatchGroup *grp) {
+    P.dev->bat_shadow = false;
+    if (prec == RBS_PREC_FP32 && P.dev->mixed && P.dev->whole()) {
+        DeviceState *own = P.dev;
+        const int rc = on_shadow(P, err, [&] { return device_batch_start(P, bcols, xcols, k, prec, more, err, grp); });
+        own->bat_shadow = rc == RBS_OK;
+        return rc;
+    }
     DeviceState &D = *P.dev;
     if (k < 1 || k > 128 || (prec != RBS_PREC_FP64 && !D.mixed)) {
         err = "batch: k must be in [1, 128]; FP32 and mixed batches need a plan with FP32 copies";
@@ -1623,6 +1633,10 @@ int device_batch_next(Plan &P, int *more, std::string &err) {
 }
 
 int device_batch_finish(Plan &P, int *iters, double *corr, std::string &err) {
+    if (P.dev->bat_shadow) {
+        P.dev->bat_shadow = false;
+        return on_shadow(P, err, [&] { return device_batch_finish(P, iters, corr, err); });
+    }
     DeviceState &D = *P.dev;
     if (iters) *iters = D.bat_iters;
     if (corr) *corr = D.bat_corr;
@@ -1895,8 +1909,7 @@ int upload_blocks(Plan &P, std::string &err) {
 
 }  // namespace
 
-int device_build(Plan &P, std::string &err) {
-    if (P.dev) device_free(P);
+static int build_state(Plan &P, bool whole, std::string &err) {
     P.dev = new DeviceState();
     DeviceState &D = *P.dev;
     if (P.opt.device >= 0) CK(cudaSetDevice(P.opt.device));
@@ -1921,7 +1934,7 @@ int device_build(Plan &P, std::string &err) {
     int rc;
     D.wn = P.n;
     D.mixed = P.opt.mixed != 0;
-    if (wants_strips(P) && (rc = upload_strips(P, err))) return rc;
+    if (whole && wants_strips(P) && (rc = upload_strips(P, err))) return rc;
     if (!D.strip) {
         if ((rc = upload(D, D.perm, P.perm, err))) return rc;
         std::vector<int> ipos(P.perm.size());
@@ -1935,8 +1948,8 @@ int device_build(Plan &P, std::string &err) {
             if ((rc = upload(D, D.full_col, P.full_col, err))) return rc;
             if ((rc = upload(D, D.full_val, P.full_val, err))) return rc;
         }
-        if (wants_la(P) && (rc = upload_la(P, err))) return rc;
-        if (!D.la && (rc = upload_band(P, err))) return rc;
+        if (whole && wants_la(P) && (rc = upload_la(P, err))) return rc;
+        if (whole && !D.la && (rc = upload_band(P, err))) return rc;
     }
     if (!D.la && !D.strip && !D.band && (rc = upload_blocks(P, err))) return rc;
     {
@@ -1957,6 +1970,50 @@ int device_build(Plan &P, std::string &err) {
     if ((rc = ensure_work(P, pow2_at_least(std::max(1, std::min(P.opt.max_rhs, 128))), err))) return rc;
     CK(cudaStreamSynchronize(D.stream));
     return RBS_OK;
+}
+
+int device_build(Plan &P, std::string &err) {
+    if (P.dev) device_free(P);
+    return build_state(P, true, err);
+}
+
+// f() with the plan's block-walk state in place of its whole-matrix walk's, on
+// the same stream.
+template <typename F>
+static int on_shadow(Plan &P, std::string &err, F &&f) {
+    DeviceState *const own = P.dev;
+    if (!own->shadow) {
+        const int rc = build_state(P, false, err);
+        own->shadow = P.dev;
+        if (rc) {
+            device_free(P);
+            own->shadow = nullptr;
+            P.dev = own;
+            return rc;
+        }
+    }
+    DeviceState &S = *own->shadow;
+    P.dev = &S;
+    const cudaStream_t st = S.stream;
+    const bool owns = S.own_stream;
+    S.stream = own->stream;
+    S.own_stream = own->own_stream;
+    if (own->profile && S.bev.empty()) {
+        S.bev.resize(2 * P.blocks.size());
+        for (auto &e : S.bev) cudaEventCreate(&e);
+    }
+    S.profile = own->profile;
+    S.bms.assign(P.blocks.size(), 0.0);
+    S.bsolves = 0;
+    const int rc = f();
+    for (size_t b = 0; b < S.bms.size() && b < own->bms.size(); ++b) own->bms[b] += S.bms[b];
+    own->bsolves += S.bsolves;
+    own->last_iters = S.last_iters;
+    own->last_corr = S.last_corr;
+    S.stream = st;
+    S.own_stream = owns;
+    P.dev = own;
+    return rc;
 }
 
 int device_profile(Plan &P, int enable, std::string &err) {
@@ -2173,6 +2230,13 @@ int device_tune(Plan &P, std::string &err) {
 
 void device_free(Plan &P) {
     if (!P.dev) return;
+    if (DeviceState *own = P.dev; own->shadow) {
+        if (own->stream) cudaStreamSynchronize(own->stream);
+        P.dev = own->shadow;
+        own->shadow = nullptr;
+        device_free(P);
+        P.dev = own;
+    }
     DeviceState &D = *P.dev;
     if (D.stream) cudaStreamSynchronize(D.stream);
     pipe_release(D);
@@ -2228,7 +2292,18 @@ void device_free(Plan &P) {
     P.dev = nullptr;
 }
 
-long long device_bytes(const Plan &P) { return P.dev ? P.dev->bytes : 0; }
+long long device_bytes(const Plan &P) {
+    return P.dev ? P.dev->bytes + (P.dev->shadow ? P.dev->shadow->bytes : 0) : 0;
+}
+
+void device_walk(const Plan &P, std::vector<int> &out) {
+    out = {0, 0};
+    if (!P.dev) return;
+    const DeviceState &D = *P.dev;
+    if (D.la) out = {1, 3};  // gather, walk, scatter
+    else if (D.strip) out = {2, 1};
+    else if (D.band) out = {3, D.band_dir ? 1 : 3};
+}
 
 int device_set_stream(Plan &P, void *stream, std::string &err) {
     if (!P.dev) {
@@ -2252,6 +2327,10 @@ int device_set_stream(Plan &P, void *stream, std::string &err) {
 
 int device_sync(Plan &P, std::string &err) {
     DeviceState &D = *P.dev;
+    if (D.shadow) {  // asynchronous FP32 solves
+        const int rc = on_shadow(P, err, [&] { return device_sync(P, err); });
+        if (rc) return rc;
+    }
     CK(cudaMemcpyAsync(D.h_status, D.status, sizeof(int), cudaMemcpyDeviceToHost, D.stream));
     CK(cudaStreamSynchronize(D.stream));
     if (D.pipe.cout) CK(cudaStreamSynchronize(D.pipe.cout));  // asynchronous host-array solves' downloads
@@ -2286,6 +2365,8 @@ int device_solve(Plan &P, const double *d_b, double *d_x, int k, int ld, int pre
         err = "plan was built without FP32 copies (options.mixed = 0)";
         return RBS_ERR_UNSUPPORTED;
     }
+    if (prec == RBS_PREC_FP32 && P.dev->whole())
+        return on_shadow(P, err, [&] { return device_solve(P, d_b, d_x, k, ld, prec, sync, stats, err); });
     DeviceState &D = *P.dev;
     int iters = 0;
     double corr = 0;
@@ -2329,6 +2410,8 @@ int device_solve(Plan &P, const double *d_b, double *d_x, int k, int ld, int pre
 }
 
 int device_finish(Plan &P, rbs_stats *stats, int k, int prec, std::string &err) {
+    if (prec == RBS_PREC_FP32 && P.dev->whole() && P.dev->shadow)
+        return on_shadow(P, err, [&] { return device_finish(P, stats, k, prec, err); });
     DeviceState &D = *P.dev;
     int rc = device_sync(P, err);
     if (rc == RBS_OK && D.profile && prec != RBS_PREC_MIXED && k <= 128) {

@@ -42,7 +42,7 @@ def test_band_factors(n, lam, band, sub):
 def test_batch_and_saved_plan(tmp_path):
     systems = [rbs.gen_lower_csr(rbs.GEN_BAND_POISSON, n=n, lam=8, band=64, seed=70 + n) for n in (40, 1500, 7, 900)]
     plan, offs = rbs.batch_analyse(systems, substitution=rbs.FORWARD, fmt=rbs.FMT_CSR)
-    assert len(plan.export("la_dim")) == 10 and plan.info().kernels[rbs.K_LEVEL] == 1
+    assert len(plan.export("la_dim")) == 10 and plan.export("walk")[0] == 1
     b = rbs.gen_uniform(9, int(offs[-1]))
     x = solve(plan, b)
     for (rp, ci, va), a, e in zip(systems, offs[:-1], offs[1:]):
