@@ -104,6 +104,7 @@ struct DeviceState {
     // whose rounding depends on the order of every sum; built on the first one
     DeviceState *shadow = nullptr;
     bool bat_shadow = false;  // the batch in flight runs there
+    bool lean = false;        // a shadow: FP32 pools and vectors only
     bool whole() const { return la || strip || band; }
     int wn = 0;  // positions of the work vectors (rows, or more with padding)
     int *la_queue = nullptr;  // one segment counter per column
@@ -276,13 +277,13 @@ int ensure_work(Plan &P, int K, std::string &err) {
             if ((rc = alloc(D, D.ex64.buf[i], (size_t)D.strip_pub * (K + 1), err))) return undo(rc);
             if (D.mixed && (rc = alloc(D, D.ex32.buf[i], (size_t)D.strip_pub * (K + 1), err))) return undo(rc);
         }
-    } else {
+    } else if (!D.lean) {
         if ((rc = alloc(D, D.bw64, cnt, err))) return undo(rc);
         if ((rc = alloc(D, D.xw64, cnt, err))) return undo(rc);
     }
     if (D.mixed) {
-        if ((rc = alloc(D, D.b64keep, cnt, err))) return undo(rc);
-        if ((rc = alloc(D, D.x64acc, cnt, err))) return undo(rc);
+        if (!D.lean && (rc = alloc(D, D.b64keep, cnt, err))) return undo(rc);
+        if (!D.lean && (rc = alloc(D, D.x64acc, cnt, err))) return undo(rc);
         if ((rc = alloc(D, D.bw32, cnt, err))) return undo(rc);
         if ((rc = alloc(D, D.xw32, cnt, err))) return undo(rc);
     }
@@ -295,7 +296,8 @@ int ensure_work(Plan &P, int K, std::string &err) {
         }
         D.ex64.dirty[0] = D.ex64.dirty[1] = D.ex32.dirty[0] = D.ex32.dirty[1] = K + 1;  // filled before use
     } else {
-        k_fill<double><<<grid_for((long long)cnt, 256, D.num_sms), 256, 0, D.stream>>>(D.xw64, (long long)cnt,
+        if (!D.lean)
+            k_fill<double><<<grid_for((long long)cnt, 256, D.num_sms), 256, 0, D.stream>>>(D.xw64, (long long)cnt,
                                                                                         sent64_host());
         if (D.mixed)
             k_fill<float><<<grid_for((long long)cnt, 256, D.num_sms), 256, 0, D.stream>>>(D.xw32, (long long)cnt,
@@ -1835,11 +1837,15 @@ int upload_band(Plan &P, std::string &err) {
 // The blocks' pools and per-kernel layouts (the block walk).
 int upload_blocks(Plan &P, std::string &err) {
     DeviceState &D = *P.dev;
-    ensure_lc(P);
+    for (const ExecBlock &B : P.blocks)
+        if (B.tri && B.kernel == RBS_K_LEVEL && B.lvl_var == LVL_LC) {
+            ensure_lc(P);
+            break;
+        }
     int rc;
     if ((rc = upload(D, D.rp, P.rp_pool, err))) return rc;
     if ((rc = upload(D, D.col, P.col_pool, err))) return rc;
-    if ((rc = upload(D, D.val, P.val_pool, err))) return rc;
+    if (!D.lean && (rc = upload(D, D.val, P.val_pool, err))) return rc;
     if ((rc = upload(D, D.lvl, P.lvl_pool, err))) return rc;
     if ((rc = upload(D, D.map, P.map_pool, err))) return rc;
     if ((rc = upload(D, D.rows, P.rows_pool, err))) return rc;
@@ -1847,8 +1853,8 @@ int upload_blocks(Plan &P, std::string &err) {
         const auto v32 = to_f32(P.val_pool);
         if ((rc = upload(D, D.val32, v32, err))) return rc;
     }
-    if ((rc = upload(D, D.band_coef, P.band_coef, err))) return rc;
-    if ((rc = upload(D, D.band_inv, P.band_inv, err))) return rc;
+    if (!D.lean && (rc = upload(D, D.band_coef, P.band_coef, err))) return rc;
+    if (!D.lean && (rc = upload(D, D.band_inv, P.band_inv, err))) return rc;
     {
         // every triangle with a band layout may run the band scan (the tuner
         // switches kernels after this point), so size for all of them
@@ -1867,7 +1873,7 @@ int upload_blocks(Plan &P, std::string &err) {
         if ((rc = upload(D, D.band_inv32, i32, err))) return rc;
     }
     if ((rc = upload(D, D.ell_col, P.ell_col, err))) return rc;
-    if ((rc = upload(D, D.ell_val, P.ell_val, err))) return rc;
+    if (!D.lean && (rc = upload(D, D.ell_val, P.ell_val, err))) return rc;
     {
         std::vector<EllChunk> ec(P.ell_chunks.size() / 4);
         std::memcpy(ec.data(), P.ell_chunks.data(), ec.size() * sizeof(EllChunk));
@@ -1883,7 +1889,7 @@ int upload_blocks(Plan &P, std::string &err) {
                 for (long long e = B.ca_lo; e < B.ca_hi; ++e) c16[(size_t)e] = (short)P.ca_col[(size_t)e];
         if ((rc = upload(D, D.ca_col16, c16, err))) return rc;
     }
-    if ((rc = upload(D, D.ca_val, P.ca_val, err))) return rc;
+    if (!D.lean && (rc = upload(D, D.ca_val, P.ca_val, err))) return rc;
     if (D.mixed) {
         const auto c32 = to_f32(P.ca_val);
         if ((rc = upload(D, D.ca_val32, c32, err))) return rc;
@@ -1896,7 +1902,7 @@ int upload_blocks(Plan &P, std::string &err) {
         std::vector<LcChunk> tab(P.lc_tab.size() / LC_TAB_INTS);
         std::memcpy(tab.data(), P.lc_tab.data(), tab.size() * sizeof(LcChunk));
         if ((rc = upload(D, D.lc_tab, tab, err))) return rc;
-        if ((rc = upload(D, D.lc_rec64, P.lc_rec64, err))) return rc;
+        if (!D.lean && (rc = upload(D, D.lc_rec64, P.lc_rec64, err))) return rc;
         if (D.mixed && (rc = upload(D, D.lc_rec32, P.lc_rec32, err))) return rc;
         std::vector<LcSeg> segs(P.lc_segs.size() / 3);
         for (size_t q = 0; q < segs.size(); ++q)
@@ -1912,6 +1918,7 @@ int upload_blocks(Plan &P, std::string &err) {
 static int build_state(Plan &P, bool whole, std::string &err) {
     P.dev = new DeviceState();
     DeviceState &D = *P.dev;
+    D.lean = !whole;
     if (P.opt.device >= 0) CK(cudaSetDevice(P.opt.device));
     CK(cudaGetDevice(&D.device));
     CK(cudaDeviceGetAttribute(&D.num_sms, cudaDevAttrMultiProcessorCount, D.device));
@@ -1940,10 +1947,12 @@ static int build_state(Plan &P, bool whole, std::string &err) {
         std::vector<int> ipos(P.perm.size());
         for (size_t p = 0; p < P.perm.size(); ++p) ipos[(size_t)P.perm[p]] = (int)p;
         if ((rc = upload(D, D.ipos, ipos, err))) return rc;
-        if ((rc = upload(D, D.inv, P.inv_diag, err))) return rc;
+        if (!D.lean && (rc = upload(D, D.inv, P.inv_diag, err))) return rc;
         if (D.mixed) {
             const auto i32 = to_f32(P.inv_diag);
             if ((rc = upload(D, D.inv32, i32, err))) return rc;
+        }
+        if (D.mixed && !D.lean) {
             if ((rc = upload(D, D.full_rp, P.full_rp, err))) return rc;
             if ((rc = upload(D, D.full_col, P.full_col, err))) return rc;
             if ((rc = upload(D, D.full_val, P.full_val, err))) return rc;
