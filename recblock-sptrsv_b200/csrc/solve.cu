@@ -57,6 +57,7 @@ struct DeviceState {
     float *band_coef32 = nullptr, *band_inv32 = nullptr;
     double *band_maps = nullptr, *band_states = nullptr; // scratch of the band scan (f64 or f32), kcap columns
     size_t band_maps1 = 1, band_states1 = 1;             // ... elements per column
+    std::vector<char> band_dominant;                     // per block: every row of its band layout is dominant
     int *ell_col = nullptr;
     double *ell_val = nullptr;
     float *ell_val32 = nullptr;
@@ -658,6 +659,23 @@ int syncfree_grid(const DeviceState &D) {
     return per_sm * D.num_sms;
 }
 
+// Whether sum |a_d| * |1/l| <= 1 in every row of a band layout (its maps then
+// never grow, band.cuh; 1e-12 for the rounding of the sum and the inverse).
+bool band_rows_dominant(const double *coef, const double *inv, size_t rows, int W) {
+    constexpr size_t kRows = 1 << 16;
+    std::atomic<bool> ok{true};
+    parallel_for((rows + kRows - 1) / kRows, [&](size_t g) {
+        bool all = true;
+        for (size_t r = g * kRows; r < std::min(rows, (g + 1) * kRows); ++r) {
+            double sum = 0;
+            for (int d = 0; d < W; ++d) sum += std::fabs(coef[r * W + d]);
+            all = all && sum * std::fabs(inv[r]) <= 1.0 + 1e-12;  // false for a NaN
+        }
+        if (!all) ok = false;
+    });
+    return ok;
+}
+
 // Band-scan triangle, or the whole matrix (see band.cuh): one launch over all
 // K right-hand sides; row p of column c at p * rs + c * cs of bb and xx.
 template <typename VT, int W, typename BT>
@@ -681,7 +699,8 @@ int run_band(Plan &P, const ExecBlock &B, const BT *bb, BT *xx, long long rs, lo
     int *flags = reinterpret_cast<int *>(states);
     CK(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)K * (nblk + 1), st));
     k_band_onepass<VT, W, BT><<<dim3(nblk, K), BAND_T, smem, st>>>(coef, binv, bb, rs, cs, B.m, B.band_c, nch, maps, flags,
-                                                                xx, D.status, P.opt.spin_limit);
+                                                                xx, D.status, P.opt.spin_limit,
+                                                                D.band || D.band_dominant[(size_t)B.index]);
     return RBS_OK;
 }
 
@@ -1760,9 +1779,10 @@ int upload_strips(Plan &P, std::string &err) {
 }
 
 // Band layout of the whole matrix, when the cost model gave every triangle
-// with off-diagonal entries to the band scan and no row reaches further than
-// 8 positions back across the triangles either (D.band stays false
-// otherwise).  Row r is row r % C of chunk r / C, as in a triangle's layout.
+// with off-diagonal entries to the band scan, no row reaches further than 8
+// positions back across the triangles either, and every row is dominant
+// (D.band stays false otherwise: the block walk's scans start anew in every
+// triangle).  Row r is row r % C of chunk r / C, as in a triangle's layout.
 int upload_band(Plan &P, std::string &err) {
     DeviceState &D = *P.dev;
     if (P.opt.select != RBS_SELECT_AUTO || P.blocks.size() < 2) return RBS_OK;
@@ -1821,6 +1841,7 @@ int upload_band(Plan &P, std::string &err) {
         if (!f) fwd = 0;
         if (!r) bwd = 0;
     });
+    if (!band_rows_dominant(coef.data(), inv.data(), slots, W)) return RBS_OK;
     D.band_dir = fwd ? 1 : bwd ? -1 : 0;
     int rc;
     if ((rc = upload(D, D.band_coef, coef, err)) || (rc = upload(D, D.band_inv, inv, err))) return rc;
@@ -1859,8 +1880,12 @@ int upload_blocks(Plan &P, std::string &err) {
         // every triangle with a band layout may run the band scan (the tuner
         // switches kernels after this point), so size for all of them
         size_t maps = 1, states = 1;
+        D.band_dominant.assign(P.blocks.size(), 0);
         for (const ExecBlock &B : P.blocks)
             if (B.tri && B.band_w > 0) {
+                D.band_dominant[(size_t)B.index] =
+                    band_rows_dominant(P.band_coef.data() + B.band_off, P.band_inv.data() + B.band_off / B.band_w,
+                                       (size_t)B.band_nch * B.band_c, B.band_w);
                 maps = std::max(maps, (size_t)band_blocks(B.band_nch) * (B.band_w * B.band_w + B.band_w));
                 states = std::max(states, ((size_t)band_blocks(B.band_nch) + 1) * sizeof(int) / sizeof(double) + 1);
             }
