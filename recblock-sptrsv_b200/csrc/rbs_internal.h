@@ -401,6 +401,8 @@ int device_staging(Plan &P, size_t bytes, double *&db, double *&dx, std::string 
 int device_host_async(Plan &P, const double *b, double *x, int k, int ld, int prec, std::string &err);
 // work vectors for k right-hand sides allocated now, so solves up to that
 // width allocate nothing
+// before a plan is served as a group of several systems (device_batch_start with a BatchGroup)
+int device_for_groups(Plan &P, std::string &err);
 int device_reserve(Plan &P, int k, std::string &err);
 // Asynchronous solve of k columns on the plan's stream: bcols / xcols are
 // device tables of k column pointers (right-hand sides read, solutions

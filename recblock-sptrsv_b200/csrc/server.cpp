@@ -396,7 +396,12 @@ int add_unit(rbs_server *s, rbs_plan *plan, int count, const int *offs, int *fac
     }
     // work vectors for the batch width now: no solve of this unit grows them later
     std::string err;
-    int rc = rbs_plan_set_stream(plan, u->stream);
+    int rc = count > 1 ? rbs::device_for_groups(plan->p, err) : RBS_OK;
+    if (rc != RBS_OK) {
+        release(*u);
+        return fail(rc, "rbs_server_add_group: " + err);
+    }
+    rc = rbs_plan_set_stream(plan, u->stream);
     if (rc == RBS_OK && (rc = rbs::device_reserve(plan->p, s->max_k, err)) != RBS_OK) rbs::set_error(err);
     if (rc != RBS_OK) {
         const std::string msg = rbs_last_error();

@@ -1940,10 +1940,12 @@ int upload_blocks(Plan &P, std::string &err) {
 
 }  // namespace
 
-static int build_state(Plan &P, bool whole, std::string &err) {
+// A new device state as P.dev: whole, with the whole-matrix walk the plan's
+// structure suits; otherwise the block walk's (lean: its FP32 half).
+static int build_state(Plan &P, bool whole, bool lean, std::string &err) {
     P.dev = new DeviceState();
     DeviceState &D = *P.dev;
-    D.lean = !whole;
+    D.lean = lean;
     if (P.opt.device >= 0) CK(cudaSetDevice(P.opt.device));
     CK(cudaGetDevice(&D.device));
     CK(cudaDeviceGetAttribute(&D.num_sms, cudaDevAttrMultiProcessorCount, D.device));
@@ -2008,7 +2010,22 @@ static int build_state(Plan &P, bool whole, std::string &err) {
 
 int device_build(Plan &P, std::string &err) {
     if (P.dev) device_free(P);
-    return build_state(P, true, err);
+    return build_state(P, true, false, err);
+}
+
+// A plan served as a group of systems: its columns come from a table per
+// system, which the strip kernel's walk on the caller's columns cannot read.
+// Batched plans never take it; a block-diagonal matrix analysed as one system
+// can, and then gets the block walk's state in its place.
+int device_for_groups(Plan &P, std::string &err) {
+    if (!P.dev || !P.dev->strip) return RBS_OK;
+    DeviceState *const old = P.dev;
+    const int rc = build_state(P, false, false, err);
+    DeviceState *const fresh = P.dev;
+    P.dev = rc ? fresh : old;
+    device_free(P);
+    P.dev = rc ? old : fresh;
+    return rc;
 }
 
 // f() with the plan's block-walk state in place of its whole-matrix walk's, on
@@ -2017,7 +2034,7 @@ template <typename F>
 static int on_shadow(Plan &P, std::string &err, F &&f) {
     DeviceState *const own = P.dev;
     if (!own->shadow) {
-        const int rc = build_state(P, false, err);
+        const int rc = build_state(P, false, true, err);
         own->shadow = P.dev;
         if (rc) {
             device_free(P);
