@@ -11,7 +11,10 @@
 // not per level.  A chunk's published rows are written when it ends, and the
 // same numbers of the other exchange vector, which the next walk uses, are
 // set back to the sentinel.  Strips are handed out by a ticket and depend on
-// earlier ones only, so any residency makes progress.
+// earlier ones only, so any residency makes progress.  The ticket counts to
+// twice the strips and starts anew: its half is the walk's parity, which says
+// which of the two exchange vectors is clean, so that state is the device's
+// alone and a walk can be recorded in a graph and replayed.
 //
 // A second warp streams the records through a ring with bulk copies and, for
 // a walk on the caller's vectors (IO), gathers the right-hand sides of a
@@ -59,9 +62,9 @@ struct StripArgs {
     const VT *b;
     VT *x;
     long long gstride;
-    VT *ex, *ex_next;  // exchange of this walk and of the next, column group y at + y * published * G
+    VT *ex0, *ex1;     // exchange vectors of even and odd walks, column group y at + y * published * G
     int published;
-    int *ticket;       // one per column group, zero before the launch
+    unsigned *ticket;  // one per column group, kept from walk to walk
     int *status;
     long long limit;
 };
@@ -145,14 +148,16 @@ __global__ void __launch_bounds__(96, 4) k_tri_strip(const __grid_constant__ Str
     constexpr unsigned E = sizeof(VT), EG = E * G, BG = sizeof(BT) * G;
     constexpr unsigned rec_bytes = st_rec_bytes(W, E), b_off = (rec_bytes + 127) / 128 * 128;
     constexpr unsigned slot_bytes = st_slot_bytes<VT, W, G, IO>();
-    __shared__ int s_strip;
+    __shared__ int s_strip, s_odd;
     __shared__ __align__(8) unsigned long long mbar[3 * SLOTS + 2 * NW];  // landed, free, b landed; solved, written
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned u_ring = smem_u32(sm), u_win = u_ring + SLOTS * slot_bytes;
     const unsigned u_full = smem_u32(mbar), u_empty = u_full + 8 * SLOTS, u_b = u_empty + 8 * SLOTS;
     const unsigned u_done = u_b + 8 * SLOTS, u_out = u_done + 8 * NW;
     if (threadIdx.x == 0) {
-        s_strip = atomicAdd(a.ticket + blockIdx.y, 1);
+        const int t = (int)atomicInc(a.ticket + blockIdx.y, 2u * a.nstrip - 1);
+        s_odd = t >= a.nstrip;
+        s_strip = s_odd ? t - a.nstrip : t;
         for (int i = 0; i < 2 * SLOTS; ++i) mbar_init(mbar + i, 1);
         for (int i = 0; i < SLOTS; ++i) mbar_init(mbar + 2 * SLOTS + i, 32);
         for (int i = 0; i < 2 * NW; ++i) mbar_init(mbar + 3 * SLOTS + i, 1);
@@ -258,7 +263,8 @@ __global__ void __launch_bounds__(96, 4) k_tri_strip(const __grid_constant__ Str
     }
 
     // ---------------- the strip's warp ----------------
-    VT *ex = a.ex + (long long)blockIdx.y * a.published * G, *exn = a.ex_next + (long long)blockIdx.y * a.published * G;
+    VT *ex = (s_odd ? a.ex1 : a.ex0) + (long long)blockIdx.y * a.published * G;
+    VT *exn = (s_odd ? a.ex0 : a.ex1) + (long long)blockIdx.y * a.published * G;
     unsigned sl = u_ring, mb = u_full, par = 0;  // the chunk after the one in hand
     bool bad = false;
     VT r[G];        // remote value of this lane for the next chunk

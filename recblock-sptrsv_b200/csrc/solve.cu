@@ -90,16 +90,19 @@ struct DeviceState {
     ExecBlock band_blk{};
     int band_dir = 0;
     int strip_w = 0, strip_n = 0, strip_pub = 0;
-    int *strip_first = nullptr, *strip_ticket = nullptr, *strip_rows = nullptr;
+    int *strip_first = nullptr, *strip_rows = nullptr;
     unsigned char *strip_at = nullptr;
-    // two exchange vectors per precision, used in turn: a walk clears the
-    // other one's numbers; columns beyond its own that still hold values
+    // exchange vectors of each precision for walks of one (0) and two (1)
+    // columns per CTA, two of each, used in turn: a walk clears the other
+    // one's numbers.  Whose turn it is stands in the tickets on the device
+    // (level_strip.cuh): 128 column groups for each precision and CTA width.
     template <typename VT> struct Exchange {
-        VT *buf[2] = {nullptr, nullptr};
-        int cur = 0, dirty[2] = {0, 0};
+        VT *buf[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+        size_t size[2] = {0, 0};
     };
     Exchange<double> ex64;
     Exchange<float> ex32;
+    unsigned *strip_ticket = nullptr;
     uint32_t *strip_rec64 = nullptr, *strip_rec32 = nullptr;
     // the block walk's state beside a whole-matrix walk's: FP32 solves keep it,
     // whose rounding depends on the order of every sum; built on the first one
@@ -227,9 +230,9 @@ void free_work(DeviceState &D) {
     cudaFree(D.xw32);
     D.bw64 = D.xw64 = D.b64keep = D.x64acc = nullptr;
     D.bw32 = D.xw32 = nullptr;
-    for (int i = 0; i < 2; ++i) {
-        cudaFree(D.ex64.buf[i]);
-        cudaFree(D.ex32.buf[i]);
+    for (int i = 0; i < 4; ++i) {
+        cudaFree(D.ex64.buf[i / 2][i % 2]);
+        cudaFree(D.ex32.buf[i / 2][i % 2]);
     }
     D.ex64 = {};
     D.ex32 = {};
@@ -248,6 +251,38 @@ float sent32_host() {
     float v;
     std::memcpy(&v, &bits, 4);
     return v;
+}
+
+// Most columns of the strip kernel at one column per CTA: while every strip
+// of every column has a CTA on the GPU at once.  Wider walks take two columns
+// per CTA (1M-row grid, 32 columns: one 563, two 505, four 562 us).
+template <typename VT> int strip_single(const DeviceState &D) {
+    const int smem = D.strip_w == 2 ? st_smem<VT, 2, 1, true>() : st_smem<VT, 4, 1, true>();
+    return std::max(1LL, (long long)D.num_sms * (D.smem_sm / (smem + D.smem_reserved)) / D.strip_n);
+}
+
+// Exchange vectors for up to K columns.
+template <typename VT> int alloc_exchange(DeviceState &D, DeviceState::Exchange<VT> &X, int K, std::string &err) {
+    const int single = strip_single<VT>(D);
+    X.size[0] = (size_t)D.strip_pub * std::min(K, single);
+    X.size[1] = K > single ? (size_t)D.strip_pub * (K + 1) : 0;
+    for (int i = 0; i < 4; ++i)
+        if (X.size[i / 2]) {
+            const int rc = alloc(D, X.buf[i / 2][i % 2], X.size[i / 2], err);
+            if (rc) return rc;
+        }
+    return RBS_OK;
+}
+
+// The strip walks' exchange as before the first of them: no values, tickets 0.
+void reset_exchange(DeviceState &D) {
+    for (int i = 0; i < 4; ++i) {
+        if (const long long n = (long long)D.ex64.size[i / 2])
+            k_fill<double><<<grid_for(n, 256, D.num_sms), 256, 0, D.stream>>>(D.ex64.buf[i / 2][i % 2], n, sent64_host());
+        if (const long long n = (long long)D.ex32.size[i / 2])
+            k_fill<float><<<grid_for(n, 256, D.num_sms), 256, 0, D.stream>>>(D.ex32.buf[i / 2][i % 2], n, sent32_host());
+    }
+    cudaMemsetAsync(D.strip_ticket, 0, sizeof(unsigned) * 4 * 128, D.stream);
 }
 
 // Work vectors sized for K right-hand sides; solution vectors start filled
@@ -274,10 +309,8 @@ int ensure_work(Plan &P, int K, std::string &err) {
     };
     int rc;
     if (D.strip) {  // FP64 walks run on the caller's vectors
-        for (int i = 0; i < 2; ++i) {
-            if ((rc = alloc(D, D.ex64.buf[i], (size_t)D.strip_pub * (K + 1), err))) return undo(rc);
-            if (D.mixed && (rc = alloc(D, D.ex32.buf[i], (size_t)D.strip_pub * (K + 1), err))) return undo(rc);
-        }
+        if ((rc = alloc_exchange(D, D.ex64, K, err))) return undo(rc);
+        if (D.mixed && (rc = alloc_exchange(D, D.ex32, K, err))) return undo(rc);
     } else if (!D.lean) {
         if ((rc = alloc(D, D.bw64, cnt, err))) return undo(rc);
         if ((rc = alloc(D, D.xw64, cnt, err))) return undo(rc);
@@ -295,7 +328,7 @@ int ensure_work(Plan &P, int K, std::string &err) {
             CK(cudaMemsetAsync(D.b64keep, 0, cnt * sizeof(double), D.stream));
             CK(cudaMemsetAsync(D.bw32, 0, cnt * sizeof(float), D.stream));
         }
-        D.ex64.dirty[0] = D.ex64.dirty[1] = D.ex32.dirty[0] = D.ex32.dirty[1] = K + 1;  // filled before use
+        reset_exchange(D);
     } else {
         if (!D.lean)
             k_fill<double><<<grid_for((long long)cnt, 256, D.num_sms), 256, 0, D.stream>>>(D.xw64, (long long)cnt,
@@ -471,13 +504,8 @@ template <typename VT> int ca_group(const ExecBlock &B, int K) {
     return G;
 }
 
-// Columns per CTA of the strip kernel: one while every strip of every column
-// has a CTA on the GPU at once, two otherwise (1M-row grid, 32 columns: one
-// 563, two 505, four 562 us).
-template <typename VT> int strip_group(const DeviceState &D, int cols) {
-    const int smem = D.strip_w == 2 ? st_smem<VT, 2, 1, true>() : st_smem<VT, 4, 1, true>();
-    return cols == 1 || (long long)D.strip_n * cols <= (long long)D.num_sms * (D.smem_sm / (smem + D.smem_reserved)) ? 1 : 2;
-}
+// Columns per CTA of the strip kernel.
+template <typename VT> int strip_group(const DeviceState &D, int cols) { return cols <= strip_single<VT>(D) ? 1 : 2; }
 
 // Layout of a K-column solve's work vectors: 0 = row-interleaved (entry
 // (p, c) at p*K + c), G > 0 = grouped by column groups of G (group c/G's
@@ -921,37 +949,24 @@ int launch_strip_wg(DeviceState &D, const StripArgs<VT> &a, int groups, std::str
     return RBS_OK;
 }
 
-// The arguments that both kinds of walk share, for `cols` columns in groups
-// of G: the exchange vectors change places, and one that still holds values
-// (of a wider walk, or a failed one) is cleared first.
+// The arguments that both kinds of walk share, for columns in groups of G.
 template <typename VT>
-int strip_args(Plan &P, StripArgs<VT> &a, int cols, int G, std::string &err) {
+StripArgs<VT> strip_args(Plan &P, int G) {
     DeviceState &D = *P.dev;
-    auto &X = Pools<VT>::ex(D);
-    const int groups = (cols + G - 1) / G, used = groups * G;
+    const auto &X = Pools<VT>::ex(D);
+    StripArgs<VT> a{};
     a.rec = reinterpret_cast<const unsigned char *>(Pools<VT>::striprec(D));
     a.first = D.strip_first;
     a.nstrip = D.strip_n;
     a.rows = D.strip_rows;
     a.rows_at = D.strip_at;
+    a.ex0 = X.buf[G - 1][0];
+    a.ex1 = X.buf[G - 1][1];
     a.published = D.strip_pub;
-    a.ticket = D.strip_ticket;
+    a.ticket = D.strip_ticket + ((sizeof(VT) == 8 ? 0 : 2) + G - 1) * 128;
     a.status = D.status;
     a.limit = wait_limit(P);
-    const int other = X.cur ^ 1;
-    for (int i = 0; i < 2; ++i)
-        if (X.dirty[i] > (i == X.cur ? 0 : used)) {
-            const long long cnt = (long long)D.strip_pub * (D.kcap + 1);
-            k_fill<VT><<<grid_for(cnt, 256, D.num_sms), 256, 0, D.stream>>>(X.buf[i], cnt, Pools<VT>::sent());
-            X.dirty[i] = 0;
-        }
-    a.ex = X.buf[X.cur];
-    a.ex_next = X.buf[other];
-    X.dirty[X.cur] = used;
-    X.dirty[other] = 0;
-    X.cur = other;
-    CK(cudaMemsetAsync(D.strip_ticket, 0, sizeof(int) * (size_t)groups, D.stream));
-    return RBS_OK;
+    return a;
 }
 
 // Walk on the work vectors in strip order (the FP32 sweeps of refinement).
@@ -959,9 +974,7 @@ template <typename VT>
 int launch_strip(Plan &P, int K, std::string &err) {
     DeviceState &D = *P.dev;
     const int G = K == 1 ? 1 : strip_group<VT>(D, K), groups = K / G;
-    StripArgs<VT> a{};
-    int rc = strip_args<VT>(P, a, K, G, err);
-    if (rc) return rc;
+    StripArgs<VT> a = strip_args<VT>(P, G);
     a.b = Pools<VT>::bw(D);
     a.x = Pools<VT>::xw(D);
     a.gstride = (long long)D.wn * G;
@@ -981,9 +994,8 @@ int solve_strip(Plan &P, const double *b, double *x, const double *const *bcols,
             CK(cudaEventRecord(D.bev[2 * B.index], D.stream));
             if (B.index) CK(cudaEventRecord(D.bev[2 * B.index + 1], D.stream));
         }
-    StripArgs<VT> a{};
-    int rc = strip_args<VT>(P, a, k, G, err);
-    if (rc) return rc;
+    StripArgs<VT> a = strip_args<VT>(P, G);
+    int rc;
     a.b64 = b;
     a.x64 = x;
     a.bcols = bcols;
@@ -1739,7 +1751,7 @@ int upload_strips(Plan &P, std::string &err) {
     if ((rc = upload(D, D.perm, perm, err)) || (rc = upload(D, D.ipos, ipos, err)) ||
         (rc = upload(D, D.strip_first, H.first, err)) || (rc = upload(D, D.strip_rec64, H.rec, err)) ||
         (rc = upload(D, D.strip_rows, H.rows_sorted, err)) || (rc = upload(D, D.strip_at, H.rows_at, err)) ||
-        (rc = alloc(D, D.strip_ticket, 128, err)))
+        (rc = alloc(D, D.strip_ticket, 4 * 128, err)))
         return rc;
     if (D.mixed) {
         const int nch = H.first.back();
@@ -2396,7 +2408,7 @@ int device_sync(Plan &P, std::string &err) {
             k_fill<float><<<grid_for((long long)cnt, 256, D.num_sms), 256, 0, D.stream>>>(
                 D.xw32, (long long)cnt, sent32_host());
         D.xw_dirty64 = D.xw_dirty32 = false;
-        D.ex64.dirty[0] = D.ex64.dirty[1] = D.ex32.dirty[0] = D.ex32.dirty[1] = D.kcap + 1;
+        if (D.strip) reset_exchange(D);
         CK(cudaStreamSynchronize(D.stream));
         err = "a device wait exceeded its poll budget (dependency never produced)";
         return RBS_ERR_TIMEOUT;
