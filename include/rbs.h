@@ -144,7 +144,11 @@ int rbs_plan_sync(rbs_plan *plan);
 int rbs_plan_set_stream(rbs_plan *plan, void *stream);
 /* Allocate the plan's work vectors for k (1..128) right-hand sides now, so
  * later solves of up to k columns allocate and free no device memory (no
- * counterpart in the reference, which allocates inside its solver). */
+ * counterpart in the reference, which allocates inside its solver).  Where
+ * FP32 solves need device state of their own (RBS_SELECT_AUTO plans built
+ * with options.mixed whose FP64 solves run on one kernel for the whole matrix)
+ * it is built here too; without this call the first RBS_PREC_FP32 solve builds
+ * it, which takes about as long as an analysis and cannot be captured. */
 int rbs_plan_reserve(rbs_plan *plan, int k);
 int rbs_plan_info_get(const rbs_plan *plan, rbs_plan_info *info);
 

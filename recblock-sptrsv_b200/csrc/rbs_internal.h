@@ -228,6 +228,41 @@ struct StripHost {
     bulk_vector<uint32_t> rec;  // FP64 records (the FP32 ones are made from them on the device)
 };
 
+// A plan's device state.  A thread that runs a solve on a plan's other state
+// (DevView) sees that one in its place; every other thread sees the plan's own.
+struct DevSlot {
+    DeviceState *own = nullptr;
+    DeviceState *get() const;
+    DevSlot &operator=(DeviceState *d) {
+        own = d;
+        return *this;
+    }
+    operator DeviceState *() const { return get(); }
+    DeviceState *operator->() const { return get(); }
+    DeviceState &operator*() const { return *get(); }
+};
+struct DevView {
+    DevView(const DevSlot &slot, DeviceState *state) : slot_(&slot), state_(state), outer_(current()) { current() = this; }
+    ~DevView() { current() = outer_; }
+    DevView(const DevView &) = delete;
+    DevView &operator=(const DevView &) = delete;
+
+private:
+    friend struct DevSlot;
+    static DevView *&current() {
+        static thread_local DevView *v = nullptr;
+        return v;
+    }
+    const DevSlot *slot_;
+    DeviceState *state_;
+    DevView *outer_;
+};
+inline DeviceState *DevSlot::get() const {
+    for (const DevView *v = DevView::current(); v; v = v->outer_)
+        if (v->slot_ == this) return v->state_;
+    return own;
+}
+
 struct Plan {
     int n = 0, nnz = 0, lv = 0, sub = 0, nlevel = 0, sum_block = 0, step = 0;
     rbs_options opt{};
@@ -280,7 +315,7 @@ struct Plan {
     bulk_vector<int> full_col;
     bulk_vector<double> full_val;
 
-    DeviceState *dev = nullptr;
+    DevSlot dev;
     // reference-format export cache (export_reference); exports of one plan
     // from several threads at once are not supported
     mutable std::shared_ptr<const RefPack> ref_pack;

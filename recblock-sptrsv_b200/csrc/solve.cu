@@ -105,8 +105,9 @@ struct DeviceState {
     unsigned *strip_ticket = nullptr;
     uint32_t *strip_rec64 = nullptr, *strip_rec32 = nullptr;
     // the block walk's state beside a whole-matrix walk's: FP32 solves keep it,
-    // whose rounding depends on the order of every sum; built on the first one
-    DeviceState *shadow = nullptr;
+    // whose rounding depends on the order of every sum; built by
+    // device_reserve, or else by the first such solve
+    std::atomic<DeviceState *> shadow{nullptr};
     bool bat_shadow = false;  // the batch in flight runs there
     bool lean = false;        // a shadow: FP32 pools and vectors only
     bool whole() const { return la || strip || band; }
@@ -1593,6 +1594,41 @@ int batch_end_k(Plan &P, double *const *xcols, int k, const GroupCols &gx, std::
 
 }  // namespace
 
+template <typename F> static int on_shadow(Plan &P, std::string &err, F &&f);
+
+namespace {
+
+// Work vectors for K right-hand sides, and what the block walks of up to K
+// build on their first run: descriptors, row lists.
+template <typename VT>
+int reserve_walks(Plan &P, int K, std::string &err) {
+    for (int q = 1; q <= K; q <<= 1) {
+        const int GL = plan_group<VT>(P, q);
+        LevelDesc *ld = nullptr;
+        CaDesc *cd = nullptr;
+        CsfDesc *ed = nullptr;
+        int rc = RBS_OK;
+        RBS_FOR_K(q, rc = (level_descs<VT, KC>(P, ld, err)));
+        if (rc == RBS_OK) rc = ca_descs<VT>(P, cd, q, GL, err);
+        if (rc == RBS_OK && q == 1) rc = ell_descs<VT>(P, ed, err);
+        if (rc == RBS_OK && q > 1 && GL) rc = ensure_io_rows(P, err);
+        if (rc) return rc;
+    }
+    return RBS_OK;
+}
+
+int reserve_state(Plan &P, int K, std::string &err) {
+    DeviceState &D = *P.dev;
+    int rc = ensure_work(P, K, err);
+    if (rc == RBS_OK && !D.whole() && !D.lean) rc = reserve_walks<double>(P, K, err);
+    if (rc == RBS_OK && !D.whole() && D.mixed) rc = reserve_walks<float>(P, K, err);
+    if (rc) return rc;
+    CK(cudaStreamSynchronize(D.stream));
+    return RBS_OK;
+}
+
+}  // namespace
+
 int device_reserve(Plan &P, int k, std::string &err) {
     if (!P.dev) {
         err = "plan has no device state";
@@ -1602,13 +1638,12 @@ int device_reserve(Plan &P, int k, std::string &err) {
         err = "reserve: k must be in [1, 128]";
         return RBS_ERR_ARG;
     }
-    int rc = ensure_work(P, pow2_at_least(k), err);
-    if (rc) return rc;
-    CK(cudaStreamSynchronize(P.dev->stream));
-    return RBS_OK;
+    const int K = pow2_at_least(k);
+    int rc = reserve_state(P, K, err);
+    if (rc == RBS_OK && P.dev->mixed && P.dev->whole())
+        rc = on_shadow(P, err, [&] { return reserve_state(P, K, err); });
+    return rc;
 }
-
-template <typename F> static int on_shadow(Plan &P, std::string &err, F &&f);
 
 int device_batch_start(Plan &P, const double *const *bcols, double *const *xcols, int k, int prec, int *more,
                        std::string &err, const BatchGroup *grp) {
@@ -1952,10 +1987,11 @@ int upload_blocks(Plan &P, std::string &err) {
 
 }  // namespace
 
-// A new device state as P.dev: whole, with the whole-matrix walk the plan's
-// structure suits; otherwise the block walk's (lean: its FP32 half).
+static void free_state(DeviceState *d);
+
+// Fills in the new device state *P.dev: whole, with the whole-matrix walk the
+// plan's structure suits; otherwise the block walk's (lean: its FP32 half).
 static int build_state(Plan &P, bool whole, bool lean, std::string &err) {
-    P.dev = new DeviceState();
     DeviceState &D = *P.dev;
     D.lean = lean;
     if (P.opt.device >= 0) CK(cudaSetDevice(P.opt.device));
@@ -2022,7 +2058,28 @@ static int build_state(Plan &P, bool whole, bool lean, std::string &err) {
 
 int device_build(Plan &P, std::string &err) {
     if (P.dev) device_free(P);
+    P.dev = new DeviceState();
     return build_state(P, true, false, err);
+}
+
+// A block-walk state for the plan, beside the one it has.
+static int new_block_state(Plan &P, bool lean, DeviceState *&out, std::string &err) {
+    DeviceState *fresh = nullptr;
+    int rc = RBS_OK;
+    try {
+        fresh = new DeviceState();
+        DevView view(P.dev, fresh);
+        rc = build_state(P, false, lean, err);
+    } catch (const std::bad_alloc &) {
+        err = "out of host memory";
+        rc = RBS_ERR_NOMEM;
+    }
+    if (rc) {
+        if (fresh) free_state(fresh);
+        return rc;
+    }
+    out = fresh;
+    return RBS_OK;
 }
 
 // A plan served as a group of systems: its columns come from a table per
@@ -2031,13 +2088,12 @@ int device_build(Plan &P, std::string &err) {
 // can, and then gets the block walk's state in its place.
 int device_for_groups(Plan &P, std::string &err) {
     if (!P.dev || !P.dev->strip) return RBS_OK;
-    DeviceState *const old = P.dev;
-    const int rc = build_state(P, false, false, err);
-    DeviceState *const fresh = P.dev;
-    P.dev = rc ? fresh : old;
+    DeviceState *fresh = nullptr;
+    const int rc = new_block_state(P, false, fresh, err);
+    if (rc) return rc;
     device_free(P);
-    P.dev = rc ? old : fresh;
-    return rc;
+    P.dev = fresh;
+    return RBS_OK;
 }
 
 // f() with the plan's block-walk state in place of its whole-matrix walk's, on
@@ -2046,21 +2102,31 @@ template <typename F>
 static int on_shadow(Plan &P, std::string &err, F &&f) {
     DeviceState *const own = P.dev;
     if (!own->shadow) {
-        const int rc = build_state(P, false, true, err);
-        own->shadow = P.dev;
-        if (rc) {
-            device_free(P);
-            own->shadow = nullptr;
-            P.dev = own;
-            return rc;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(own->stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone) {
+            err = "the plan's first FP32 solve cannot be captured: reserve or solve once before";
+            return RBS_ERR_UNSUPPORTED;
         }
+        DeviceState *fresh = nullptr;
+        const int rc = new_block_state(P, true, fresh, err);
+        if (rc) return rc;
+        own->shadow = fresh;
     }
-    DeviceState &S = *own->shadow;
-    P.dev = &S;
-    const cudaStream_t st = S.stream;
-    const bool owns = S.own_stream;
-    S.stream = own->stream;
-    S.own_stream = own->own_stream;
+    struct Run {  // the state runs on the plan's stream, and reports to it
+        DeviceState &own, &S;
+        cudaStream_t st;
+        bool owns;
+        Run(DeviceState &o, DeviceState &s) : own(o), S(s), st(s.stream), owns(s.own_stream) {
+            S.stream = own.stream;
+            S.own_stream = own.own_stream;
+        }
+        ~Run() {
+            S.stream = st;
+            S.own_stream = owns;
+        }
+    } run(*own, *own->shadow);
+    DeviceState &S = run.S;
+    DevView view(P.dev, &S);
     if (own->profile && S.bev.empty()) {
         S.bev.resize(2 * P.blocks.size());
         for (auto &e : S.bev) cudaEventCreate(&e);
@@ -2073,9 +2139,6 @@ static int on_shadow(Plan &P, std::string &err, F &&f) {
     own->bsolves += S.bsolves;
     own->last_iters = S.last_iters;
     own->last_corr = S.last_corr;
-    S.stream = st;
-    S.own_stream = owns;
-    P.dev = own;
     return rc;
 }
 
@@ -2293,15 +2356,14 @@ int device_tune(Plan &P, std::string &err) {
 
 void device_free(Plan &P) {
     if (!P.dev) return;
-    if (DeviceState *own = P.dev; own->shadow) {
-        if (own->stream) cudaStreamSynchronize(own->stream);
-        P.dev = own->shadow;
-        own->shadow = nullptr;
-        device_free(P);
-        P.dev = own;
-    }
-    DeviceState &D = *P.dev;
+    free_state(P.dev);
+    P.dev = nullptr;
+}
+
+static void free_state(DeviceState *d) {
+    DeviceState &D = *d;
     if (D.stream) cudaStreamSynchronize(D.stream);
+    if (D.shadow) free_state(D.shadow);
     pipe_release(D);
     free_work(D);
     drop_graphs(D);
@@ -2351,12 +2413,13 @@ void device_free(Plan &P) {
     if (D.ev1) cudaEventDestroy(D.ev1);
     if (D.ev_in) cudaEventDestroy(D.ev_in);
     if (D.own_stream && D.stream) cudaStreamDestroy(D.stream);
-    delete P.dev;
-    P.dev = nullptr;
+    delete d;
 }
 
 long long device_bytes(const Plan &P) {
-    return P.dev ? P.dev->bytes + (P.dev->shadow ? P.dev->shadow->bytes : 0) : 0;
+    if (!P.dev) return 0;
+    const DeviceState *S = P.dev->shadow;
+    return P.dev->bytes + (S ? S->bytes : 0);
 }
 
 void device_walk(const Plan &P, std::vector<int> &out) {
@@ -2388,12 +2451,24 @@ int device_set_stream(Plan &P, void *stream, std::string &err) {
     return RBS_OK;
 }
 
+static int sync_own(Plan &P, std::string &err);
+
 int device_sync(Plan &P, std::string &err) {
     DeviceState &D = *P.dev;
     if (D.shadow) {  // asynchronous FP32 solves
-        const int rc = on_shadow(P, err, [&] { return device_sync(P, err); });
-        if (rc) return rc;
+        std::string err2;
+        const int rc = on_shadow(P, err2, [&] { return device_sync(P, err2); });
+        if (rc) {  // its own solves' status is still collected
+            const int own = sync_own(P, err);
+            if (own == RBS_OK) err = err2;
+            return rc;
+        }
     }
+    return sync_own(P, err);
+}
+
+static int sync_own(Plan &P, std::string &err) {
+    DeviceState &D = *P.dev;
     CK(cudaMemcpyAsync(D.h_status, D.status, sizeof(int), cudaMemcpyDeviceToHost, D.stream));
     CK(cudaStreamSynchronize(D.stream));
     if (D.pipe.cout) CK(cudaStreamSynchronize(D.pipe.cout));  // asynchronous host-array solves' downloads
