@@ -695,9 +695,10 @@ bool wants_strips(const Plan &P) {
 }
 
 void ensure_lc(Plan &P) {
+    const std::lock_guard<std::mutex> lock(P.lc_mu);  // exports and saves of one plan may come from several threads
     if (!P.lc_deferred) return;
-    P.lc_deferred = false;
     build_lc(P, P.opt, local_levels(P));
+    P.lc_deferred = false;
 }
 
 int host_bfs_levels(const int *cp, const int *ri, int m, std::vector<int> &levelPtr, std::vector<int> &item) {

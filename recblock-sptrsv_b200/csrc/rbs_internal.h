@@ -27,6 +27,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <string>
 #include <thread>
@@ -301,6 +302,7 @@ struct Plan {
     // out until they are asked for (ensure_lc); the look-ahead layout is kept
     // here from the analysis to the upload.
     bool lc_deferred = false;
+    std::mutex lc_mu;  // of the two lines above, and the records
     std::vector<char> level_better;  // per block, level_preferred (not saved)
     std::shared_ptr<LaHost> la;
     std::shared_ptr<StripHost> strip;  // the same for the strip kernel
