@@ -119,7 +119,7 @@ bool la_build(const Plan &P, LaHost &H) {
         while (cur < nseg) seg_first[(size_t)++cur] = (int)ch.size();
     }
     const size_t nch = ch.size();
-    if (nch == 0) return false;
+    if (nch == 0 || (double)nch * D.rec_bytes(8) > la_most_bytes(rp[n], n)) return false;
     auto vr = [&](int q) { return nseg > 1 ? vrow[(size_t)q] : q; };
 
     // window size: the smallest that leaves few entries outside
@@ -191,6 +191,7 @@ bool la_build(const Plan &P, LaHost &H) {
         D.nx = std::max(D.nx, (extra[c] + 7) / 8 * 8);
     }
     if (oo > INT_MAX - 65536 || D.slots(8) < LA_SLOTS_MIN) return false;
+    if ((double)nch * D.rec_bytes(8) > la_most_bytes(rp[n], n)) return false;  // with the extra terms
     const size_t recw = (size_t)D.rec_bytes(8) / 4;
     H.rec.resize(nch * recw);
     H.old.resize((size_t)oo);

@@ -57,6 +57,15 @@ static_assert(LA_XW_MIN >= (LA_AHEAD + 1) * LA_RMAX, "old values are final when 
 static_assert(LA_AUX >= (LA_AHEAD + 2) * LA_OLD, "gathered values are used before their slots are");
 constexpr int LA_SMEM = 232448 - 1024;
 constexpr int LA_THREADS = 960;  // main and helper threads at most
+// FP64 records at most: eight times the matrix's CSR (12 bytes an entry), or 16
+// MB.  A record is as large for one row as for a full chunk, so levels of a few
+// rows take many times the matrix: bands of 128 with 4 to 12 entries a row 3.8
+// to 5.4 times, a batch of 256 bands of 256 2.2 times, a band of 24 with 10
+// entries 14 times, a chain that reads its last 9 rows 31 times.
+constexpr double la_most_bytes(int nnz, int n) {
+    const double csr = 12.0 * nnz + 4.0 * (n + 1.0);
+    return 8 * csr > 16e6 ? 8 * csr : 16e6;
+}
 
 struct LaChunk {
     int lo, nr;    // processing positions [lo, lo + nr)

@@ -380,7 +380,7 @@ void ensure_lc(Plan &P);
 bool wants_strips(const Plan &P);
 // strip_build.h; false: the structure does not suit the kernel
 bool strip_build(const Plan &P, StripHost &H);
-// la_build.h; false: the structure does not suit the kernel
+// la_build.h; false: the structure does not suit the kernel, or would take too much memory
 bool la_build(const Plan &P, LaHost &H);
 
 // ilu0.cu: ILU(0) of a device CSR matrix into d_lu (A's pattern)

@@ -1730,6 +1730,18 @@ int solve_k(Plan &P, const double *b, double *x, int k, int ld, int prec, int &i
 
 namespace {
 
+// An upload of a whole-matrix walk's layout that ran out of device memory is
+// taken back (its arrays freed) and the plan keeps the block walk.
+template <typename... T>
+int take_back(DeviceState &D, int rc, long long bytes_before, std::string &err, T *&...arrays) {
+    if (rc != RBS_ERR_NOMEM) return rc;
+    ((cudaFree(arrays), arrays = nullptr), ...);
+    cudaGetLastError();  // the failed allocation's
+    D.bytes = bytes_before;
+    err.clear();
+    return RBS_OK;
+}
+
 // Builds and uploads the look-ahead layout (D.la stays false where the
 // structure does not suit it).
 int upload_la(Plan &P, std::string &err) {
@@ -2016,7 +2028,12 @@ static int build_state(Plan &P, bool whole, bool lean, std::string &err) {
     int rc;
     D.wn = P.n;
     D.mixed = P.opt.mixed != 0;
-    if (whole && wants_strips(P) && (rc = upload_strips(P, err))) return rc;
+    long long before = D.bytes;
+    if (whole && wants_strips(P)) {
+        rc = take_back(D, upload_strips(P, err), before, err, D.perm, D.ipos, D.strip_first, D.strip_rec64, D.strip_rows,
+                       D.strip_at, D.strip_ticket, D.strip_rec32, D.full_rp, D.full_col, D.full_val);
+        if (rc) return rc;
+    }
     if (!D.strip) {
         if ((rc = upload(D, D.perm, P.perm, err))) return rc;
         std::vector<int> ipos(P.perm.size());
@@ -2032,7 +2049,11 @@ static int build_state(Plan &P, bool whole, bool lean, std::string &err) {
             if ((rc = upload(D, D.full_col, P.full_col, err))) return rc;
             if ((rc = upload(D, D.full_val, P.full_val, err))) return rc;
         }
-        if (whole && wants_la(P) && (rc = upload_la(P, err))) return rc;
+        before = D.bytes;
+        if (whole && wants_la(P)) {
+            rc = take_back(D, upload_la(P, err), before, err, D.la_tab, D.la_rec64, D.la_old, D.la_segs, D.la_queue, D.la_rec32);
+            if (rc) return rc;
+        }
         if (whole && !D.la && (rc = upload_band(P, err))) return rc;
     }
     if (!D.la && !D.strip && !D.band && (rc = upload_blocks(P, err))) return rc;
