@@ -694,6 +694,17 @@ bool wants_strips(const Plan &P) {
     return any;
 }
 
+// The layouts, kept until they are uploaded; one that was refused stays
+// (empty, not ok), so that it is not tried again.
+void build_la(Plan &P) {
+    P.la = std::make_shared<LaHost>();
+    if (!la_build(P, *P.la)) *P.la = LaHost{};
+}
+void build_strips(Plan &P) {
+    P.strip = std::make_shared<StripHost>();
+    if (!strip_build(P, *P.strip)) *P.strip = StripHost{};
+}
+
 void ensure_lc(Plan &P) {
     const std::lock_guard<std::mutex> lock(P.lc_mu);  // exports and saves of one plan may come from several threads
     if (!P.lc_deferred) return;
@@ -1333,14 +1344,9 @@ int analyse_after_levels(Plan &P, int n, int nnz, int substitution, int lv, cons
     P.la.reset();
     P.strip.reset();
     P.lc_deferred = false;
-    if (!opt.host_only && wants_strips(P)) {
-        P.strip = std::make_shared<StripHost>();
-        if (!strip_build(P, *P.strip)) P.strip.reset();
-    } else if (!opt.host_only && wants_la(P)) {
-        P.la = std::make_shared<LaHost>();
-        if (!la_build(P, *P.la)) P.la.reset();
-    }
-    if (P.la || P.strip) {
+    if (!opt.host_only && wants_strips(P)) build_strips(P);
+    else if (!opt.host_only && wants_la(P)) build_la(P);
+    if ((P.la && P.la->ok) || (P.strip && P.strip->ok)) {
         P.lc_deferred = true;
         P.lc_rec64.clear();
         P.lc_rec32.clear();

@@ -378,6 +378,9 @@ bool wants_la(Plan &P);
 void ensure_lc(Plan &P);
 // analysis.cpp: whether strips are worth trying for the plan's whole walk
 bool wants_strips(const Plan &P);
+// analysis.cpp: P.la and P.strip from the two builders below
+void build_la(Plan &P);
+void build_strips(Plan &P);
 // strip_build.h; false: the structure does not suit the kernel
 bool strip_build(const Plan &P, StripHost &H);
 // la_build.h; false: the structure does not suit the kernel, or would take too much memory

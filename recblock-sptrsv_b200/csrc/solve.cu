@@ -1746,10 +1746,7 @@ int take_back(DeviceState &D, int rc, long long bytes_before, std::string &err, 
 // structure does not suit it).
 int upload_la(Plan &P, std::string &err) {
     DeviceState &D = *P.dev;
-    if (!P.la) {
-        P.la = std::make_shared<LaHost>();
-        la_build(P, *P.la);
-    }
+    if (!P.la) build_la(P);
     if (!P.la->ok) return RBS_OK;
     LaHost &H = *P.la;
     int rc;
@@ -1780,10 +1777,7 @@ int upload_la(Plan &P, std::string &err) {
 // precision, the full CSR in that order (padding rows empty).
 int upload_strips(Plan &P, std::string &err) {
     DeviceState &D = *P.dev;
-    if (!P.strip) {
-        P.strip = std::make_shared<StripHost>();
-        strip_build(P, *P.strip);
-    }
+    if (!P.strip) build_strips(P);
     if (!P.strip->ok) return RBS_OK;
     const StripHost &H = *P.strip;
     int rc;
