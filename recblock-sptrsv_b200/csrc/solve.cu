@@ -1733,12 +1733,15 @@ namespace {
 // An upload of a whole-matrix walk's layout that ran out of device memory is
 // taken back (its arrays freed) and the plan keeps the block walk.
 template <typename... T>
-int take_back(DeviceState &D, int rc, long long bytes_before, std::string &err, T *&...arrays) {
+int take_back(Plan &P, int rc, long long bytes_before, std::string &err, T *&...arrays) {
     if (rc != RBS_ERR_NOMEM) return rc;
+    DeviceState &D = *P.dev;
     ((cudaFree(arrays), arrays = nullptr), ...);
     cudaGetLastError();  // the failed allocation's
     D.bytes = bytes_before;
     err.clear();
+    P.la.reset();
+    P.strip.reset();
     return RBS_OK;
 }
 
@@ -2024,7 +2027,7 @@ static int build_state(Plan &P, bool whole, bool lean, std::string &err) {
     D.mixed = P.opt.mixed != 0;
     long long before = D.bytes;
     if (whole && wants_strips(P)) {
-        rc = take_back(D, upload_strips(P, err), before, err, D.perm, D.ipos, D.strip_first, D.strip_rec64, D.strip_rows,
+        rc = take_back(P, upload_strips(P, err), before, err, D.perm, D.ipos, D.strip_first, D.strip_rec64, D.strip_rows,
                        D.strip_at, D.strip_ticket, D.strip_rec32, D.full_rp, D.full_col, D.full_val);
         if (rc) return rc;
     }
@@ -2045,7 +2048,7 @@ static int build_state(Plan &P, bool whole, bool lean, std::string &err) {
         }
         before = D.bytes;
         if (whole && wants_la(P)) {
-            rc = take_back(D, upload_la(P, err), before, err, D.la_tab, D.la_rec64, D.la_old, D.la_segs, D.la_queue, D.la_rec32);
+            rc = take_back(P, upload_la(P, err), before, err, D.la_tab, D.la_rec64, D.la_old, D.la_segs, D.la_queue, D.la_rec32);
             if (rc) return rc;
         }
         if (whole && !D.la && (rc = upload_band(P, err))) return rc;
