@@ -383,19 +383,19 @@ static int device_factor(bool ic, const int *d_rp, const int *d_ci, const double
         return RBS_ERR_CUDA;
     cudaStream_t st = nullptr;
     cudaMemPool_t pool = nullptr;  // the per-device stream-ordered pool (allocations on st)
-    int *scratch = nullptr;  // diag[n], done[n], ticket, status, bad_row, longest row
+    int *scratch = nullptr;  // diag[n], done[n], ticket, status, bad_row, longest row, deepest level
     int rc = RBS_OK;
     if (!ck(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream") ||
         !ck(device_mem_pool(dev, pool), "memory pool") ||
-        !ck(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&scratch), sizeof(int) * (2 * (size_t)n + 4), pool, st),
+        !ck(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&scratch), sizeof(int) * (2 * (size_t)n + 5), pool, st),
             "cudaMallocFromPoolAsync"))
         rc = RBS_ERR_CUDA;
     int *diag = scratch, *done = scratch + n, *ticket = scratch + 2 * (size_t)n, *status = ticket + 1,
         *bad = ticket + 2;
-    int h[4] = {0, 0, 0, 0};
+    int h[5] = {0, 0, 0, 0, 0};
     bool short_rows = false;
     if (rc == RBS_OK) {
-        const int bad0[4] = {0, 0, 0x7fffffff, 0};
+        const int bad0[5] = {0, 0, 0x7fffffff, 0, 0};
         bool ok = ck(cudaMemcpyAsync(ticket, bad0, sizeof(bad0), cudaMemcpyHostToDevice, st), "memcpy");
         if (ok) {
             const int g = (n + 255) / 256 < sms * 8 ? (n + 255) / 256 : sms * 8;
@@ -415,6 +415,47 @@ static int device_factor(bool ic, const int *d_rp, const int *d_ci, const double
             rc = RBS_ERR_STRUCTURE;
         }
     }
+    // rows in dependency-level order (level of row i = 1 + the largest level
+    // of the rows of its lower part; all of them precede i), ascending inside
+    // a level: the rows in flight at a time span whole levels, and every
+    // dependency of a row has an earlier ticket
+    int *order = nullptr, *lv = nullptr;  // order[n]; levels, sorted levels, rows, ticket
+    void *tmp = nullptr;
+    if (rc == RBS_OK) {
+        const size_t N = (size_t)n;
+        bool ok = ck(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&order), sizeof(int) * N, pool, st),
+                     "cudaMallocFromPoolAsync") &&
+                  ck(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&lv), sizeof(int) * (3 * N + 1), pool, st),
+                     "cudaMallocFromPoolAsync") &&
+                  ck(cudaMemsetAsync(lv, 0xff, sizeof(int) * N, st), "memset") &&
+                  ck(cudaMemsetAsync(lv + 3 * N, 0, sizeof(int), st), "memset");
+        int *rows = ok ? lv + 2 * N : nullptr;
+        if (ok) {
+            // 32 rows a warp; more warps than fit only queue.  Up to 64 times the
+            // rows of the factor kernels are in flight, so that a chain's last one
+            // waits several times as long as there: eight times their poll budget.
+            const long long limit = 8 * std::min<long long>(opt.spin_limit, 1LL << 56);
+            const long long ctas = ((long long)n + 255) / 256;
+            k_row_levels<<<(unsigned)(ctas < sms * 8 ? ctas : sms * 8), 256, 0, st>>>(d_rp, d_ci, n, lv, rows, lv + 3 * N, status,
+                                                                                ticket + 4, limit);
+            ok = ck(cudaGetLastError(), "launch") &&
+                 ck(cudaMemcpyAsync(h, ticket, sizeof(h), cudaMemcpyDeviceToHost, st), "memcpy") &&
+                 ck(cudaStreamSynchronize(st), "sync");
+        }
+        if (ok && (h[1] & RBS_STATUS_TIMEOUT)) {
+            // an order by unfinished levels could put a row before one it waits for
+            err = std::string(who) + ": a dependency wait of the level search exceeded its poll budget";
+            rc = RBS_ERR_TIMEOUT;
+        } else if (ok) {
+            int bits = 1;
+            while (bits < 31 && (h[4] >> bits)) ++bits;
+            size_t bytes = 0;
+            ok = ck(cub::DeviceRadixSort::SortPairs(nullptr, bytes, lv, lv + N, rows, order, n, 0, bits, st), "sort") &&
+                 ck(cudaMallocFromPoolAsync(&tmp, bytes ? bytes : 1, pool, st), "cudaMallocFromPoolAsync") &&
+                 ck(cub::DeviceRadixSort::SortPairs(tmp, bytes, lv, lv + N, rows, order, n, 0, bits, st), "sort");
+        }
+        if (!ok) rc = RBS_ERR_CUDA;
+    }
     if (rc == RBS_OK) {
         // a factor that overlaps the matrix's own values is computed in place
         const double *v1 = d_val + nnz, *l1 = d_lu + nnz;
@@ -429,40 +470,6 @@ static int device_factor(bool ic, const int *d_rp, const int *d_ci, const double
         } else {
             ok = ck(cudaMemsetAsync(done, 0, sizeof(int) * (size_t)n, st), "memset") &&
                  ck(cudaMemcpyAsync(d_lu, d_val, sizeof(double) * (size_t)nnz, cudaMemcpyDeviceToDevice, st), "memcpy");
-        }
-        if (!ok) rc = RBS_ERR_CUDA;
-    }
-    // rows in dependency-level order (level of row i = 1 + the largest level
-    // of the rows of its lower part; all of them precede i), ascending inside
-    // a level: the rows in flight at a time span whole levels, and every
-    // dependency of a row has an earlier ticket
-    int *order = nullptr, *lv = nullptr;  // order[n]; levels, sorted levels, rows, ticket, deepest
-    void *tmp = nullptr;
-    if (rc == RBS_OK) {
-        const size_t N = (size_t)n;
-        bool ok = ck(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&order), sizeof(int) * N, pool, st),
-                     "cudaMallocFromPoolAsync") &&
-                  ck(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&lv), sizeof(int) * (3 * N + 2), pool, st),
-                     "cudaMallocFromPoolAsync") &&
-                  ck(cudaMemsetAsync(lv, 0xff, sizeof(int) * N, st), "memset") &&
-                  ck(cudaMemsetAsync(lv + 3 * N, 0, 2 * sizeof(int), st), "memset");
-        int *rows = ok ? lv + 2 * N : nullptr, top = 0;
-        if (ok) {
-            // 32 rows a warp; more warps than fit only queue
-            const long long ctas = ((long long)n + 255) / 256;
-            k_row_levels<<<(unsigned)(ctas < sms * 8 ? ctas : sms * 8), 256, 0, st>>>(d_rp, d_ci, n, lv, rows, lv + 3 * N, status,
-                                                                                lv + 3 * N + 1, opt.spin_limit);
-            ok = ck(cudaGetLastError(), "launch") &&
-                 ck(cudaMemcpyAsync(&top, lv + 3 * N + 1, sizeof(int), cudaMemcpyDeviceToHost, st), "memcpy") &&
-                 ck(cudaStreamSynchronize(st), "sync");
-        }
-        if (ok) {
-            int bits = 1;
-            while (bits < 31 && (top >> bits)) ++bits;
-            size_t bytes = 0;
-            ok = ck(cub::DeviceRadixSort::SortPairs(nullptr, bytes, lv, lv + N, rows, order, n, 0, bits, st), "sort") &&
-                 ck(cudaMallocFromPoolAsync(&tmp, bytes ? bytes : 1, pool, st), "cudaMallocFromPoolAsync") &&
-                 ck(cub::DeviceRadixSort::SortPairs(tmp, bytes, lv, lv + N, rows, order, n, 0, bits, st), "sort");
         }
         if (!ok) rc = RBS_ERR_CUDA;
     }
