@@ -58,7 +58,9 @@ __device__ __forceinline__ void st_release_int(int *p, int v) {
 }
 
 // diagonal position of every row; the row pointer must be valid and the
-// columns in range and ascending (checked before any of them is used)
+// columns in range and ascending (checked before any of them is used).
+// *longest: entries of the longest row, or INT_MAX when the arrays hold entries
+// before the first row or behind the last, which only the copying kernel keeps.
 __global__ void k_ilu0_diag(const int *__restrict__ rp, const int *__restrict__ ci, int n, int nnz, int *diag,
                             int *status, int *bad_row, int *longest) {
     int most = 0;
@@ -74,6 +76,7 @@ __global__ void k_ilu0_diag(const int *__restrict__ rp, const int *__restrict__ 
         if (d < 0) flag |= ILU_MISSING_DIAG;
         diag[i] = d;
         most = max(most, e - b);
+        if ((i == 0 && b != 0) || (i == n - 1 && e != nnz)) most = 0x7fffffff;
         if (flag) {
             atomicOr(status, flag);
             atomicMin(bad_row, i);

@@ -2,7 +2,8 @@
 returns RBS_ERR_TIMEOUT before any factor kernel is launched (the output is
 untouched), and the next call with the default limit gives the serial factor
 bit for bit.  The matrix is a chain, whose 32-row groups wait for one another
-in turn, so that most of them poll far more often than the limit set here."""
+in turn, so that most of them poll far more often than the limit set here.
+And ILU(0) of arrays that hold more entries than the matrix."""
 import numpy as np
 import pytest
 
@@ -35,3 +36,16 @@ def test_level_search_out_of_polls(ic):
     assert bool((lu == 7.0).all())
     run(*d, lu)
     assert np.array_equal(lu.cpu().numpy(), ref(rp, ci, va))
+
+
+@pytest.mark.parametrize("before,behind", [(3, 0), (0, 5), (2, 2)])
+def test_entries_outside_the_rows_are_copied(before, behind):
+    # arrays larger than the matrix: the factor's other entries are the matrix's own
+    rp, ci, va = chain(5000, False)
+    pad = lambda a, v: np.concatenate([np.full(before, v, a.dtype), a, np.full(behind, v, a.dtype)])
+    d = [torch.tensor(a, device="cuda") for a in (rp + before, pad(ci, 0), pad(va, -2.5))]
+    lu = torch.full_like(d[2], 7.0)
+    rbs.ilu0_device(*d, lu)
+    assert np.array_equal(lu.cpu().numpy(), pad(oracle.ilu0_csr(rp, ci, va), -2.5))
+    rbs.ilu0_device(*d, d[2])
+    assert torch.equal(d[2], lu)
