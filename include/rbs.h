@@ -140,7 +140,11 @@ int rbs_solve_async(rbs_plan *plan, const double *d_b, double *d_x, int k, int l
 int rbs_solve_host_async(rbs_plan *plan, const double *b, double *x, int k, int ld, int prec);
 int rbs_plan_sync(rbs_plan *plan);
 
-/* cudaStream_t passed as void* (NULL = the plan's own stream). */
+/* cudaStream_t passed as void* (NULL = the plan's own stream).  The plan's own
+ * stream is a non-blocking one: a caller whose arrays are still being written
+ * on another stream waits for that first, or sets that stream here.  (Work
+ * queued on the legacy default stream is waited for where a solve on device
+ * arrays writes x from its first microseconds on.) */
 int rbs_plan_set_stream(rbs_plan *plan, void *stream);
 /* Allocate the plan's work vectors for k (1..128) right-hand sides now, so
  * later solves of up to k columns allocate and free no device memory (no

@@ -200,7 +200,8 @@ int rbs_solve(rbs_plan *plan, const double *d_b, double *d_x, int k, int ld, int
     int rc = check_solve_args(plan, d_b, d_x, k, ld, prec);
     if (rc) return rc;
     std::string err;
-    rc = rbs::device_solve(plan->p, d_b, d_x, k, ld, prec, true, stats, err);
+    rc = rbs::device_after_default(plan->p, prec, err);
+    if (rc == RBS_OK) rc = rbs::device_solve(plan->p, d_b, d_x, k, ld, prec, true, stats, err);
     if (rc) return fail(rc, err);
     return RBS_OK;
 }
@@ -210,7 +211,8 @@ int rbs_solve_async(rbs_plan *plan, const double *d_b, double *d_x, int k, int l
     if (rc) return rc;
     if (prec == RBS_PREC_MIXED) return rbs_solve(plan, d_b, d_x, k, ld, prec, nullptr);
     std::string err;
-    rc = rbs::device_solve(plan->p, d_b, d_x, k, ld, prec, false, nullptr, err);
+    rc = rbs::device_after_default(plan->p, prec, err);
+    if (rc == RBS_OK) rc = rbs::device_solve(plan->p, d_b, d_x, k, ld, prec, false, nullptr, err);
     if (rc) return fail(rc, err);
     return RBS_OK;
 }

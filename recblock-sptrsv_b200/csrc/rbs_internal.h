@@ -425,6 +425,13 @@ int plan_load(Plan &P, const char *path, std::string &err);
 // solve.cu
 int device_build(Plan &P, std::string &err);
 void device_free(Plan &P);
+// Before a solve on a caller's device arrays: on the plan's own stream, a walk
+// that writes its first solutions a few microseconds after its launch (strips,
+// band scan, in FP64) comes after the work already queued on the legacy default
+// stream, where a caller may have filled b or x just before.  Other walks write
+// x in their last kernel.  While a blocking stream is being captured the legacy
+// stream may not be used, and the solve goes ahead.
+int device_after_default(Plan &P, int prec, std::string &err);
 int device_solve(Plan &P, const double *d_b, double *d_x, int k, int ld, int prec, bool sync,
                  rbs_stats *stats, std::string &err);
 int device_sync(Plan &P, std::string &err);

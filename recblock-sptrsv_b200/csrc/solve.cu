@@ -2511,6 +2511,21 @@ static int sync_own(Plan &P, std::string &err) {
 
 void *device_stream(Plan &P) { return P.dev ? (void *)P.dev->stream : nullptr; }
 
+int device_after_default(Plan &P, int prec, std::string &err) {
+    if (!P.dev) return RBS_OK;
+    DeviceState &D = *P.dev;
+    if (!D.own_stream || prec != RBS_PREC_FP64 || !(D.strip || (D.band && D.band_dir))) return RBS_OK;
+    // asked before the event is recorded: a record that a capture forbids would invalidate the capture
+    cudaStreamCaptureStatus cap;
+    if (cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return RBS_OK;
+    }
+    if (cudaEventRecord(D.ev_in, cudaStreamLegacy) == cudaSuccess) CK(cudaStreamWaitEvent(D.stream, D.ev_in, 0));
+    else cudaGetLastError();
+    return RBS_OK;
+}
+
 int device_solve(Plan &P, const double *d_b, double *d_x, int k, int ld, int prec, bool sync, rbs_stats *stats,
                  std::string &err) {
     if (!P.dev) {
@@ -2527,14 +2542,6 @@ int device_solve(Plan &P, const double *d_b, double *d_x, int k, int ld, int pre
     int iters = 0;
     double corr = 0;
     int rc = RBS_OK;
-    // On the plan's own stream, work already queued on the default stream
-    // (a caller filling b or x just before) comes first: the whole-matrix
-    // walks write the first solutions a few microseconds after their launch.
-    // While another stream's capture forbids the event, the solve goes ahead.
-    if (D.own_stream) {
-        if (cudaEventRecord(D.ev_in, cudaStreamLegacy) == cudaSuccess) CK(cudaStreamWaitEvent(D.stream, D.ev_in, 0));
-        else cudaGetLastError();
-    }
     CK(cudaEventRecord(D.ev0, D.stream));
     for (int c0 = 0; c0 < k && rc == RBS_OK; c0 += 128) {
         int kk = std::min(128, k - c0);
