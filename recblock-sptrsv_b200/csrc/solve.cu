@@ -984,17 +984,22 @@ int launch_strip(Plan &P, int K, std::string &err) {
     return G == 1 ? launch_strip_wg<VT, 4, 1, false>(D, a, groups, err) : launch_strip_wg<VT, 4, 2, false>(D, a, groups, err);
 }
 
+// Per-block events of a profiled walk in one launch, which follows: every other
+// block's first, so that only the launch lies between the first block's.
+cudaError_t profile_whole(Plan &P) {
+    DeviceState &D = *P.dev;
+    cudaError_t e = cudaSuccess;
+    for (size_t i = 2; i < 2 * P.blocks.size() && e == cudaSuccess; ++i) e = cudaEventRecord(D.bev[i], D.stream);
+    return e == cudaSuccess ? cudaEventRecord(D.bev[0], D.stream) : e;
+}
+
 // Walk on the caller's columns (b + c * ld and x + c * ld, or the tables).
 template <typename VT>
 int solve_strip(Plan &P, const double *b, double *x, const double *const *bcols, double *const *xcols, int k, int ld,
                 std::string &err) {
     DeviceState &D = *P.dev;
     const int G = strip_group<VT>(D, k), groups = (k + G - 1) / G;
-    if (D.profile)
-        for (const ExecBlock &B : P.blocks) {
-            CK(cudaEventRecord(D.bev[2 * B.index], D.stream));
-            if (B.index) CK(cudaEventRecord(D.bev[2 * B.index + 1], D.stream));
-        }
+    if (D.profile) CK(profile_whole(P));
     StripArgs<VT> a = strip_args<VT>(P, G);
     int rc;
     a.b64 = b;
@@ -1387,11 +1392,7 @@ void scatter_out(DeviceState &D, int n, VT *xw, int k, double *x, int ld, double
 template <typename VT>
 int solve_band(Plan &P, const double *b, double *x, int k, int ld, std::string &err) {
     DeviceState &D = *P.dev;
-    if (D.profile)
-        for (const ExecBlock &B : P.blocks) {
-            CK(cudaEventRecord(D.bev[2 * B.index], D.stream));
-            if (B.index) CK(cudaEventRecord(D.bev[2 * B.index + 1], D.stream));
-        }
+    if (D.profile) CK(profile_whole(P));
     const long long o = D.band_dir > 0 ? 0 : P.n - 1;
     int rc = run_band_any<VT, double>(P, D.band_blk, b + o, x + o, D.band_dir, ld, k, err);
     if (rc) return rc;
