@@ -11,7 +11,7 @@
 // consecutive rows (a chunk); a CTA scans its BAND_T chunk maps in shared
 // memory (Kogge-Stone) and publishes their total; the state entering the
 // CTA is its predecessors' totals applied in order to the zero state (where
-// every row is diagonally dominant, composed pairwise across the CTA's threads
+// products of the maps stay bounded, composed pairwise across the CTA's threads
 // first); each thread applies the composition of its CTA's earlier chunks to
 // that state and replays its rows from there.  CTAs take their place in the
 // chain from a ticket, so every predecessor a CTA waits for is already running
@@ -22,15 +22,16 @@
 // Band coefficients are stored chunk-interleaved (row i of chunk j at
 // [(i*nch + j)*W]) so the threads of a warp read consecutive addresses.
 // When every triangle of a plan is such a chain, no row reaches further back
-// across them either and every row is dominant, the whole matrix is one scan
+// across them either and the maps stay bounded, the whole matrix is one scan
 // on the caller's own vectors (1M rows of bandwidth 3: 195 -> 49 us; eight
 // triangles and seven squares in a row before).
 // For diagonally dominant rows every ||M_p||_inf <= 1, so composed maps stay
 // bounded and the scan is as stable as substitution.  Other rows' maps may
 // grow: over a few thousand rows (one CTA of a triangle) products of moderate
-// growth stay finite, but over a whole chain they overflow (ratio 1.01: after
-// 71,000 rows), and infinity times the zero state is NaN although every
-// solution is finite.  Hence the two conditions on dominance above.
+// growth stay finite, but over a whole chain they overflow (ratio 1.02: after
+// 36,000 rows), and infinity times a zero state is NaN although every solution
+// is finite.  Hence the condition on the maps, checked when the device state
+// is built (band_maps_bounded).
 #pragma once
 
 #include "kernels.cuh"
@@ -211,14 +212,14 @@ __device__ __forceinline__ void band_apply_pairwise(const VT *agg, int cnt, VT *
 // ticket first, then one flag per CTA; zeroed before the launch).  Row p of
 // column c is element p * rs + c * cs of b and x: a work vector's, or the
 // caller's own (BT = double, rs = 1 or -1) where the rows are solved in the
-// caller's order or its reverse.  dominant: the totals of several CTAs may be
-// composed with one another (every row is dominant).  Waits are bounded: after
+// caller's order or its reverse.  bounded: the totals of several CTAs may be
+// composed with one another.  Waits are bounded: after
 // `limit` polls a CTA raises RBS_STATUS_TIMEOUT and goes on.
 template <typename VT, int W, typename BT>
 __global__ void __launch_bounds__(BAND_T) k_band_onepass(const VT *__restrict__ coef, const VT *__restrict__ inv,
                                                          const BT *__restrict__ b, long long rs, long long cs, int m,
                                                          int C, int nch, VT *__restrict__ agg, int *flags, BT *x,
-                                                         int *status, long long limit, int dominant) {
+                                                         int *status, long long limit, int bounded) {
     extern __shared__ unsigned char smem_raw[];
     VT *sm = reinterpret_cast<VT *>(smem_raw);
     __shared__ VT s_state[W];
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(BAND_T) k_band_onepass(const VT *__restrict__ 
                 if (it > 16) __nanosleep(64);
             }
         }
-        if (W <= 4 && dominant) {  // wider maps do not fit the registers
+        if (W <= 4 && bounded) {  // wider maps do not fit the registers
             if constexpr (W <= 4) band_apply_pairwise<VT, W>(agg + (long long)base * E, cnt, sm, s_state, s0);
         } else {
             __syncthreads();

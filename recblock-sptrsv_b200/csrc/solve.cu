@@ -57,7 +57,7 @@ struct DeviceState {
     float *band_coef32 = nullptr, *band_inv32 = nullptr;
     double *band_maps = nullptr, *band_states = nullptr; // scratch of the band scan (f64 or f32), kcap columns
     size_t band_maps1 = 1, band_states1 = 1;             // ... elements per column
-    std::vector<char> band_dominant;                     // per block: every row of its band layout is dominant
+    std::vector<char> band_bounded;                      // per block: its band layout's maps (band_maps_bounded)
     int *ell_col = nullptr;
     double *ell_val = nullptr;
     float *ell_val32 = nullptr;
@@ -688,21 +688,91 @@ int syncfree_grid(const DeviceState &D) {
     return per_sm * D.num_sms;
 }
 
-// Whether sum |a_d| * |1/l| <= 1 in every row of a band layout (its maps then
-// never grow, band.cuh; 1e-12 for the rounding of the sum and the inverse).
-bool band_rows_dominant(const double *coef, const double *inv, size_t rows, int W) {
-    constexpr size_t kRows = 1 << 16;
+// Whether the maps of m rows in a band layout (nch chunks of C rows) may be
+// composed freely: the CTAs' totals have norm 1 at most, so that no product of
+// them grows, and no product the scan inside a CTA forms exceeds 1,000.  Rows
+// that are all dominant (sum |a_d| * |1/l| <= 1) are such maps; of others the
+// products themselves are formed, as the kernel does (the transpose of a chain
+// with dominant rows has rows that are not, and its products decay).
+template <int W>
+bool band_maps_bounded(const double *coef, const double *inv, int m, int C, int nch) {
+    constexpr double kOne = 1.0 + 1e-12, kMost = 1e3;  // 1e-12: rounding of sums and inverses
     std::atomic<bool> ok{true};
-    parallel_for((rows + kRows - 1) / kRows, [&](size_t g) {
-        bool all = true;
-        for (size_t r = g * kRows; r < std::min(rows, (g + 1) * kRows); ++r) {
-            double sum = 0;
-            for (int d = 0; d < W; ++d) sum += std::fabs(coef[r * W + d]);
-            all = all && sum * std::fabs(inv[r]) <= 1.0 + 1e-12;  // false for a NaN
+    const auto all = [&](size_t count, auto &&holds) {  // false also for a NaN
+        ok = true;
+        parallel_for(count, [&](size_t g) {
+            if (ok && !holds((int)g)) ok = false;
+        });
+        return ok.load();
+    };
+    const size_t rows = (size_t)C * nch;
+    constexpr size_t kRows = 1 << 16;
+    if (all((rows + kRows - 1) / kRows, [&](int g) {
+            bool d = true;
+            for (size_t r = (size_t)g * kRows; r < std::min(rows, (g + 1) * kRows); ++r) {
+                double sum = 0;
+                for (int q = 0; q < W; ++q) sum += std::fabs(coef[r * W + q]);
+                d = d && sum * std::fabs(inv[r]) <= kOne;
+            }
+            return d;
+        }))
+        return true;
+    struct Map {
+        double v[W][W];
+    };
+    const auto norm_within = [](const Map &M, double most) {
+        for (int r = 0; r < W; ++r) {
+            double s = 0;
+            for (int q = 0; q < W; ++q) s += std::fabs(M.v[r][q]);
+            if (!(s <= most)) return false;
         }
-        if (!all) ok = false;
+        return true;
+    };
+    return all((size_t)band_blocks(nch), [&](int o) {
+        std::vector<Map> M((size_t)BAND_T), N((size_t)BAND_T);
+        for (int t = 0; t < BAND_T; ++t) {
+            Map &A = M[(size_t)t];
+            for (int r = 0; r < W; ++r)
+                for (int q = 0; q < W; ++q) A.v[r][q] = r == q;
+            const int j = o * BAND_T + t;
+            for (int i = 0; j < nch && i < std::min(C, m - j * C); ++i) {
+                const size_t at = (size_t)i * nch + j;
+                double top[W];
+                for (int q = 0; q < W; ++q) {
+                    double s = 0;
+                    for (int d = 0; d < W; ++d) s += coef[at * W + d] * A.v[d][q];
+                    top[q] = -inv[at] * s;
+                }
+                for (int d = W - 1; d > 0; --d)
+                    for (int q = 0; q < W; ++q) A.v[d][q] = A.v[d - 1][q];
+                for (int q = 0; q < W; ++q) A.v[0][q] = top[q];
+            }
+            if (!norm_within(A, kMost)) return false;
+        }
+        for (int off = 1; off < BAND_T; off <<= 1) {
+            for (int t = off; t < BAND_T; ++t) {
+                const Map &A = M[(size_t)t], &B = M[(size_t)(t - off)];
+                Map &R = N[(size_t)t];
+                for (int r = 0; r < W; ++r)
+                    for (int q = 0; q < W; ++q) {
+                        double s = 0;
+                        for (int d = 0; d < W; ++d) s += A.v[r][d] * B.v[d][q];
+                        R.v[r][q] = s;
+                    }
+                if (!norm_within(R, kMost)) return false;
+            }
+            std::copy(N.begin() + off, N.end(), M.begin() + off);
+        }
+        return o + 1 == band_blocks(nch) || norm_within(M[(size_t)BAND_T - 1], kOne);  // the last total is not used
     });
-    return ok;
+}
+bool band_maps_bounded(const double *coef, const double *inv, const ExecBlock &B) {
+    switch (B.band_w) {
+    case 1: return band_maps_bounded<1>(coef, inv, B.m, B.band_c, B.band_nch);
+    case 2: return band_maps_bounded<2>(coef, inv, B.m, B.band_c, B.band_nch);
+    case 4: return band_maps_bounded<4>(coef, inv, B.m, B.band_c, B.band_nch);
+    default: return band_maps_bounded<8>(coef, inv, B.m, B.band_c, B.band_nch);
+    }
 }
 
 // Band-scan triangle, or the whole matrix (see band.cuh): one launch over all
@@ -729,7 +799,7 @@ int run_band(Plan &P, const ExecBlock &B, const BT *bb, BT *xx, long long rs, lo
     CK(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)K * (nblk + 1), st));
     k_band_onepass<VT, W, BT><<<dim3(nblk, K), BAND_T, smem, st>>>(coef, binv, bb, rs, cs, B.m, B.band_c, nch, maps, flags,
                                                                 xx, D.status, P.opt.spin_limit,
-                                                                D.band || D.band_dominant[(size_t)B.index]);
+                                                                D.band || D.band_bounded[(size_t)B.index]);
     return RBS_OK;
 }
 
@@ -1837,7 +1907,7 @@ int upload_strips(Plan &P, std::string &err) {
 
 // Band layout of the whole matrix, when the cost model gave every triangle
 // with off-diagonal entries to the band scan, no row reaches further than 8
-// positions back across the triangles either, and every row is dominant
+// positions back across the triangles either, and the rows' maps stay bounded
 // (D.band stays false otherwise: the block walk's scans start anew in every
 // triangle).  Row r is row r % C of chunk r / C, as in a triangle's layout.
 int upload_band(Plan &P, std::string &err) {
@@ -1898,7 +1968,7 @@ int upload_band(Plan &P, std::string &err) {
         if (!f) fwd = 0;
         if (!r) bwd = 0;
     });
-    if (!band_rows_dominant(coef.data(), inv.data(), slots, W)) return RBS_OK;
+    if (!band_maps_bounded(coef.data(), inv.data(), B)) return RBS_OK;
     D.band_dir = fwd ? 1 : bwd ? -1 : 0;
     int rc;
     if ((rc = upload(D, D.band_coef, coef, err)) || (rc = upload(D, D.band_inv, inv, err))) return rc;
@@ -1937,12 +2007,11 @@ int upload_blocks(Plan &P, std::string &err) {
         // every triangle with a band layout may run the band scan (the tuner
         // switches kernels after this point), so size for all of them
         size_t maps = 1, states = 1;
-        D.band_dominant.assign(P.blocks.size(), 0);
+        D.band_bounded.assign(P.blocks.size(), 0);
         for (const ExecBlock &B : P.blocks)
             if (B.tri && B.band_w > 0) {
-                D.band_dominant[(size_t)B.index] =
-                    band_rows_dominant(P.band_coef.data() + B.band_off, P.band_inv.data() + B.band_off / B.band_w,
-                                       (size_t)B.band_nch * B.band_c, B.band_w);
+                D.band_bounded[(size_t)B.index] =
+                    band_maps_bounded(P.band_coef.data() + B.band_off, P.band_inv.data() + B.band_off / B.band_w, B);
                 maps = std::max(maps, (size_t)band_blocks(B.band_nch) * (B.band_w * B.band_w + B.band_w));
                 states = std::max(states, ((size_t)band_blocks(B.band_nch) + 1) * sizeof(int) / sizeof(double) + 1);
             }

@@ -1,4 +1,4 @@
-"""Banded chains whose rows are not diagonally dominant: products of their
+"""Banded chains whose maps grow: products of their
 maps over the whole chain overflow although the solutions are finite, so the
 band scan must not form them.  The right-hand side is a unit vector 1,000 rows
 before the end of the substitution (all earlier solutions are zero, the last
@@ -55,8 +55,26 @@ def test_growing_chain(coefs, select, sub):
     assert walk == 0  # not one scan over the whole matrix
 
 
+@pytest.mark.parametrize("bw", [1, 2, 3, 8])
+@pytest.mark.parametrize("n", [5000, 60001, 1000000])
+def test_transposed_dominant_chain_keeps_the_whole_scan(n, bw):
+    # rows of the transpose are not dominant, their products decay all the same
+    rp, ci, va = rbs.gen_lower_csr(rbs.GEN_CHAIN, n=n, chain_bw=bw, seed=n + bw)
+    L = oracle.transpose(rp, ci, va)
+    off = np.abs(L[2]).copy()
+    first = L[0][:-1]
+    assert bw == 1 or (np.add.reduceat(off, first) > 2 * off[first]).any()
+    plan = rbs.analyse(rp, ci, va, substitution=rbs.BACKWARD, lv=1, fmt=rbs.FMT_CSC)
+    assert n == 5000 or plan.export("walk")[0] == 3
+    b = rbs.gen_uniform(3, n)
+    x = torch.full((n,), float("nan"), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    plan.solve(torch.tensor(b, device="cuda"), x)
+    assert rel_err(x.cpu().numpy(), oracle.sptrsv_csr(*L, rbs.BACKWARD, b)) <= 1e-12
+
+
 @pytest.mark.parametrize("coefs,walk", [((1.0,), 3), ((0.5, 0.25, 0.25), 3), ((1.0 + 1e-9,), 0)])
-def test_dominant_rows_keep_the_whole_scan(coefs, walk):
+def test_rows_at_the_limit_of_dominance(coefs, walk):
     n = 60001
     rp, ci, va = chain(n, coefs)
     plan = rbs.analyse(rp, ci, va, substitution=rbs.FORWARD, lv=1, fmt=rbs.FMT_CSR)
