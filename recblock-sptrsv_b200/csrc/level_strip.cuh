@@ -50,12 +50,12 @@ struct StripArgs {
     const unsigned char *rec;
     const int *first;  // first chunk of every strip, and the end
     int nstrip;
-    // IO: the caller's columns, b + c * ld (or the table bcols[c]), c < k
+    // IO: the caller's columns, b + c * ldb and x + c * ld (or the tables'), c < k
     const double *b64;
     double *x64;
     const double *const *bcols;
     double *const *xcols;
-    int ld, k;
+    int ldb, ld, k;
     const int *rows;             // per chunk its original rows ascending (-1 last)
     const unsigned char *rows_at;  // and the position in the chunk of each
     // otherwise: work vectors in strip order, column group y at + y * gstride
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(96, 4) k_tri_strip(const __grid_constant__ Str
         if constexpr (IO) {
 #pragma unroll
             for (int g = 0; g < G; ++g)
-                bp[g] = col0 + g >= a.k ? nullptr : a.bcols ? a.bcols[col0 + g] : a.b64 + (long long)(col0 + g) * a.ld;
+                bp[g] = col0 + g >= a.k ? nullptr : a.bcols ? a.bcols[col0 + g] : a.b64 + (long long)(col0 + g) * a.ldb;
         }
         StripList L;
         auto ahead = [&](int j) {  // chunk j's lists into L2: their latency there is what a chunk has to hide

@@ -1054,6 +1054,19 @@ int launch_strip(Plan &P, int K, std::string &err) {
     return G == 1 ? launch_strip_wg<VT, 4, 1, false>(D, a, groups, err) : launch_strip_wg<VT, 4, 2, false>(D, a, groups, err);
 }
 
+// Whether a column of x shares elements with a column of b other than its own:
+// such a right-hand side is read before any solution is written (the walks on
+// the caller's columns write x as they go; x the same array as b is theirs too,
+// as every element of b is read before its solution replaces it).
+bool overlaps(const double *b, const double *x, int n, int k, int ld) {
+    const long long d = (long long)(reinterpret_cast<intptr_t>(x) - reinterpret_cast<intptr_t>(b)), el = sizeof(double);
+    if (d == 0) return false;
+    const long long step = el * ld, span = el * n, m0 = d / step;  // x's column c begins d bytes after b's
+    for (long long m = m0 - 1; m <= m0 + 1; ++m)
+        if (std::llabs(m) < k && std::llabs(d - m * step) < span) return true;
+    return false;
+}
+
 // Per-block events of a profiled walk in one launch, which follows: every other
 // block's first, so that only the launch lies between the first block's.
 cudaError_t profile_whole(Plan &P) {
@@ -1068,6 +1081,19 @@ template <typename VT>
 int solve_strip(Plan &P, const double *b, double *x, const double *const *bcols, double *const *xcols, int k, int ld,
                 std::string &err) {
     DeviceState &D = *P.dev;
+    int ldb = ld;
+    if (b && overlaps(b, x, P.n, k, ld)) {  // read from a copy
+        if (!D.b64keep) {
+            const long long before = D.bytes;
+            const int rc = alloc(D, D.b64keep, (size_t)D.wn * D.kcap, err);
+            if (rc) return rc;
+            D.work_bytes += D.bytes - before;
+        }
+        ldb = P.n;
+        const size_t row = sizeof(double) * (size_t)P.n;
+        CK(cudaMemcpy2DAsync(D.b64keep, row, b, sizeof(double) * (size_t)ld, row, (size_t)k, cudaMemcpyDeviceToDevice, D.stream));
+        b = D.b64keep;
+    }
     const int G = strip_group<VT>(D, k), groups = (k + G - 1) / G;
     if (D.profile) CK(profile_whole(P));
     StripArgs<VT> a = strip_args<VT>(P, G);
@@ -1076,6 +1102,7 @@ int solve_strip(Plan &P, const double *b, double *x, const double *const *bcols,
     a.x64 = x;
     a.bcols = bcols;
     a.xcols = xcols;
+    a.ldb = ldb;
     a.ld = ld;
     a.k = k;
     if (D.strip_w == 2)
@@ -1478,7 +1505,7 @@ template <int K>
 int solve_fp64(Plan &P, const double *b, double *x, int k, int ld, std::string &err) {
     DeviceState &D = *P.dev;
     if (D.strip) return solve_strip<double>(P, b, x, nullptr, nullptr, k, ld, err);
-    if (D.band && D.band_dir) return solve_band<double>(P, b, x, k, ld, err);
+    if (D.band && D.band_dir && !overlaps(b, x, P.n, k, ld)) return solve_band<double>(P, b, x, k, ld, err);
     const int GL = plan_group<double>(P, K);
     if (K > 1 && GL && !D.la) {
         int rc = ensure_io_rows(P, err);
