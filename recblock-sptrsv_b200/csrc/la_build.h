@@ -89,34 +89,43 @@ bool la_build(const Plan &P, LaHost &H) {
     std::vector<int> vrow;  // position -> virtual row (identity for one segment)
     if (nseg > 1) vrow.resize((size_t)n);
     {
-        int cur = -1, v0 = 0, prev = -1;
-        for (const Range &g : ranges) {
-            while (cur < g.seg) {
-                seg_first[(size_t)++cur] = (int)ch.size();
-                v0 = 0;
-                prev = -1;
-            }
-            for (int a = g.lo; a < g.hi;) {
-                int nr = 0, used = 0;
-                while (a + nr < g.hi && nr < NM) {
-                    const int p = a + nr;
-                    int e = rp[p + 1] - rp[p] - 1;  // early entries: columns ascend, the late ones are at the end
-                    for (int k = rp[p + 1] - 1; prev >= 0 && k >= rp[p] && col[k] >= prev; --k) e -= col[k] != p;
-                    const int need = std::max(1, (e + Q - 1) / Q);
-                    if (need > NH || need > 24) return false;  // a long row: another kernel's work
-                    if (used + need > NH) break;
-                    used += need;
-                    ++nr;
+        std::vector<size_t> range0((size_t)nseg + 1, ranges.size());  // first range of every segment
+        for (size_t i = ranges.size(); i-- > 0;) range0[(size_t)ranges[i].seg] = i;
+        for (size_t q = (size_t)nseg; q-- > 0;) range0[q] = std::min(range0[q], range0[q + 1]);
+        std::vector<std::vector<Ch>> parts((size_t)nseg);
+        std::atomic<bool> ok{true};
+        parallel_for((size_t)nseg, [&](size_t q) {  // segments on host threads
+            int v0 = 0, prev = -1;
+            for (size_t i = range0[q]; i < range0[q + 1] && ok; ++i) {
+                const Range &g = ranges[i];
+                for (int a = g.lo; a < g.hi;) {
+                    int nr = 0, used = 0;
+                    while (a + nr < g.hi && nr < NM) {
+                        const int p = a + nr;
+                        int e = rp[p + 1] - rp[p] - 1;  // early entries: columns ascend, the late ones are at the end
+                        for (int k = rp[p + 1] - 1; prev >= 0 && k >= rp[p] && col[k] >= prev; --k) e -= col[k] != p;
+                        const int need = std::max(1, (e + Q - 1) / Q);
+                        if (need > NH || need > 24) {  // a long row: another kernel's work
+                            ok = false;
+                            return;
+                        }
+                        if (used + need > NH) break;
+                        used += need;
+                        ++nr;
+                    }
+                    parts[q].push_back({a, nr, v0, g.seg, prev});
+                    if (nseg > 1)
+                        for (int t = 0; t < nr; ++t) vrow[(size_t)(a + t)] = v0 + t;
+                    prev = a;
+                    v0 += nr;
+                    a += nr;
                 }
-                ch.push_back({a, nr, v0, g.seg, prev});
-                if (nseg > 1)
-                    for (int t = 0; t < nr; ++t) vrow[(size_t)(a + t)] = v0 + t;
-                prev = a;
-                v0 += nr;
-                a += nr;
             }
-        }
-        while (cur < nseg) seg_first[(size_t)++cur] = (int)ch.size();
+        });
+        if (!ok) return false;
+        for (int q = 0; q < nseg; ++q) seg_first[(size_t)q + 1] = seg_first[(size_t)q] + (int)parts[(size_t)q].size();
+        ch.reserve((size_t)seg_first[(size_t)nseg]);
+        for (const auto &v : parts) ch.insert(ch.end(), v.begin(), v.end());
     }
     const size_t nch = ch.size();
     if (nch == 0 || (double)nch * D.rec_bytes(8) > la_most_bytes(rp[n], n)) return false;
@@ -128,15 +137,15 @@ bool la_build(const Plan &P, LaHost &H) {
     {
         std::vector<std::vector<long long>> part((nch + 255) / 256, std::vector<long long>(kNw, 0));
         parallel_for(part.size(), [&](size_t g) {
+            long long beyond[kNw] = {};  // (a row's own entry is within every window)
             for (size_t c = g * 256; c < std::min(nch, g * 256 + 256); ++c) {
                 const Ch &C = ch[c];
-                for (int p = C.lo; p < C.lo + C.nr; ++p)
-                    for (int k = rp[p]; k < rp[p + 1]; ++k) {
-                        if (col[k] == p) continue;
-                        const int d = C.v0 + C.nr - vr(col[k]);
-                        for (int w = 0; w < kNw; ++w) part[g][(size_t)w] += d > (LA_XW_MIN << w);
-                    }
+                for (int k = rp[C.lo]; k < rp[C.lo + C.nr]; ++k) {
+                    const int d = C.v0 + C.nr - vr(col[k]);
+                    for (int w = 0; w < kNw; ++w) beyond[w] += d > (LA_XW_MIN << w);
+                }
             }
+            std::copy(beyond, beyond + kNw, part[g].begin());
         });
         for (const auto &v : part)
             for (int w = 0; w < kNw; ++w) outside[(size_t)w] += v[(size_t)w];
