@@ -57,8 +57,12 @@ extern "C" {
 #define RBS_SELECT_REFERENCE 0 /* the reference's thresholds pick the method per block
                                   (recblocking_preprocess.h:472-709, 835-922); each reference
                                   method maps to this library's kernel of the same kind */
-#define RBS_SELECT_AUTO 1      /* cost model over this library's kernels */
-#define RBS_SELECT_TUNE 2      /* time the candidate kernels per block at analysis, keep the fastest */
+#define RBS_SELECT_AUTO 1      /* cost model over this library's kernels; where the whole matrix suits
+                                  one of them, an FP64 solve is one walk of that kernel, and so is
+                                  every sweep of a mixed one */
+#define RBS_SELECT_TUNE 2      /* time the candidate kernels per block at analysis, keep the fastest;
+                                  always walks the blocks one after another, so AUTO is the faster
+                                  choice where it takes one walk (rbs_plan_export "walk") */
 
 typedef struct rbs_options {
     int select;             /* RBS_SELECT_* (default AUTO) */
@@ -69,7 +73,9 @@ typedef struct rbs_options {
     int mixed;              /* 1: also build FP32 factor copies for RBS_PREC_MIXED/FP32 (default 1) */
     double ir_tol;          /* refinement stop: ||dx||/||x|| <= ir_tol (default 1e-13) */
     int ir_max_iter;        /* default 8 */
-    long long spin_limit;   /* polls before a device wait gives up (default 1<<22 with backoff) */
+    long long spin_limit;   /* polls before a device wait gives up (default 1<<22 with backoff; the
+                               whole-matrix walks by levels and by strips poll 1<<20 times at
+                               least, as they wait for copies of their own too) */
 } rbs_options;
 
 typedef struct rbs_stats {
@@ -126,7 +132,9 @@ int rbs_solve_host(rbs_plan *plan, const double *b, double *x, int k, int ld, in
                    rbs_stats *stats);
 
 /* Asynchronous variant: enqueue on the plan's stream and return.  Status of
- * the device-side checks is collected by rbs_plan_sync. */
+ * the device-side checks is collected by rbs_plan_sync.  A graph that has
+ * recorded a solve refers to the plan's work vectors: reserve the widest k
+ * first (rbs_plan_reserve), as a wider solve replaces them. */
 int rbs_solve_async(rbs_plan *plan, const double *d_b, double *d_x, int k, int ld, int prec);
 /* Asynchronous HOST-array solve (no counterpart in the reference): b is
  * uploaded on a copy stream into one of two plan-owned staging slots, solved
@@ -226,7 +234,10 @@ int rbs_server_destroy(rbs_server *server);
  * "ptr_offset", "index_offset", "dcsrindex_offset", "recblock_Ptr",
  * "recblock_Index", "recblock_Val", "recblock_dcsr_rowidx", "method", "nlv",
  * "longrow", "m_new_dcsr", "lvl_ptr", "lvl_item", "m_lv", "offset_lv",
- * "nnz_lv", "sizes", plus this library's "kernel" (RBS_K_* per block).
+ * "nnz_lv", "sizes", plus this library's "kernel" (RBS_K_* per block) and
+ * "walk": how FP64 and mixed solves run (0 block by block; in one launch over
+ * the whole matrix: 1 by levels, 2 by strips, 3 as a band scan) and the
+ * kernels of one FP64 solve of one column (0 for the block walk).
  * With dst == NULL only *count is set.  Returns RBS_ERR_ARG for an unknown
  * name or cap < count. */
 int rbs_plan_export(const rbs_plan *plan, const char *name, void *dst, long long cap,

@@ -119,9 +119,6 @@ int pick_group(double avg) {
     return 32;
 }
 
-// Kernel choice.  REFERENCE maps each reference method to this library's
-// kernel of the same kind; AUTO uses a latency/bandwidth cost model of the
-// B200 (constants measured on a B200 with bench.py).
 // Whether a single-CTA level kernel is the better choice for a triangle once
 // its levels may run on the look-ahead kernel (the whole-matrix walk; the
 // block walk keeps select_kernel's choice).  nseg: independent systems of a
@@ -138,6 +135,9 @@ bool level_preferred(const ExecBlock &b, const std::vector<int> &lvl_sizes, int 
     return passes * 0.12 + bytes / (180e3 * ctas) + 4.0 < (double)b.nlv * 0.9 + bytes / 4.0e6 + 4.0;
 }
 
+// Kernel choice.  REFERENCE maps each reference method to this library's
+// kernel of the same kind; AUTO uses a latency/bandwidth cost model of the
+// B200 (constants measured on a B200 with bench.py).
 void select_kernel(ExecBlock &b, const rbs_options &opt, const std::vector<int> &lvl_sizes) {
     if (!b.tri) {
         if (b.nnz == 0) {
