@@ -26,12 +26,12 @@
 //
 // What bounds it: the step's chain (window write, window read, two
 // multiply-adds, subtraction, multiplication) and the instructions around it,
-// about 80 ns a step
-// for a strip alone (8,192 x 32 grid), and the steps every strip falls behind
+// about 80 ns a step for a strip alone (8,192 x 32 grid), and the steps every strip falls behind
 // the one before it (122 ns a level over 32 strips).  Measured against the
 // block walk of staged level triangles it replaces (one B200, whole solve):
-// 1024 x 1024 grid forward 945 -> 270 us, 777 x 777 backward 587 -> 202 us, 32
-// columns 1,340 -> 510 us, 64 columns 1,830 -> 864 us.  Without the fused moves
+// 1024 x 1024 grid forward 945 -> 260 us (265 with the ticket set to zero by a
+// memset before each walk), 777 x 777 backward 587 -> 199 us, 32 columns
+// 1,340 -> 512 us, 64 columns 1,830 -> 863 us.  Without the fused moves
 // (gather and scatter kernels in strip order) 32 columns took 1,255 us; asking
 // for remote values a whole chunk ahead, with chunks not shifted, 288 us for
 // one column.  Past 16 columns the caller's vectors bound it: 64-byte pieces of
