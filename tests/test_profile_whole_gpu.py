@@ -23,11 +23,13 @@ def test_first_block_is_the_launch(walk, spec):
     for _ in range(3):
         plan.solve(b, x)
     plain = min(plan.solve(b, x).ms for _ in range(20))
-    plan.profile(True)
-    plan.solve(b, x)
-    plan.profile(True)
-    stats = [plan.solve(b, x).ms for _ in range(20)]
-    ms, _, solves = plan.block_times()
-    assert solves == 20
-    assert 0 < ms[0] / 20 <= 1.25 * plain + 0.010
-    assert ms.sum() <= sum(stats)
+    first, within = [], []
+    for _ in range(20):  # the least of 20: the host may be late with a launch
+        plan.profile(True)
+        total = plan.solve(b, x).ms
+        ms, _, solves = plan.block_times()
+        assert solves == 1
+        first.append(ms[0])
+        within.append(ms.sum() <= total)
+    assert 0 < min(first) <= 1.25 * plain + 0.010
+    assert all(within)

@@ -67,14 +67,18 @@ def test_wide_and_narrow_strip_solves(mixed):
 
 
 def test_band_scan_out_of_polls():
-    # 148 CTAs start together and wait for the totals of all before them
+    # CTAs on every SM start together and wait for the totals of all before them
     L = rbs.gen_lower_csr(rbs.GEN_CHAIN, n=1000000, chain_bw=3, seed=5)
     plan = rbs.analyse(*L, substitution=rbs.FORWARD, lv=1, fmt=rbs.FMT_CSR, opts=rbs.options(spin_limit=1))
     assert plan.export("walk")[0] == 3
     b, x = torch.ones(plan.n, dtype=torch.float64, device="cuda"), torch.empty(plan.n, dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()
-    with pytest.raises(rbs.RbsError) as e:
-        plan.solve(b, x)
-    assert e.value.code == rbs.ERR_TIMEOUT
+    codes = set()
+    for _ in range(50):  # two polls may just suffice for one solve
+        try:
+            plan.solve(b, x)
+        except rbs.RbsError as e:
+            codes.add(e.code)
+    assert codes == {rbs.ERR_TIMEOUT}
     plan = rbs.analyse(*L, substitution=rbs.FORWARD, lv=1, fmt=rbs.FMT_CSR)
     check(plan, L, rbs.FORWARD, 1)
