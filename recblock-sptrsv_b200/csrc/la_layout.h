@@ -60,7 +60,7 @@ constexpr int LA_THREADS = 960;  // main and helper threads at most
 // FP64 records at most: eight times the matrix's CSR (12 bytes an entry), or 16
 // MB.  A record is as large for one row as for a full chunk, so levels of a few
 // rows take many times the matrix: bands of 128 with 4 to 12 entries a row 3.8
-// to 5.4 times, a batch of 256 bands of 256 2.2 times, a band of 24 with 10
+// to 5.4 times, a batch of 256 bands of 256 2.4 times, a band of 24 with 10
 // entries 14 times, a chain that reads its last 9 rows 31 times.
 constexpr double la_most_bytes(int nnz, int n) {
     const double csr = 12.0 * nnz + 4.0 * (n + 1.0);
