@@ -139,87 +139,22 @@ __device__ __forceinline__ void band_st_release(int *p, int v) {
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// The state after cnt totals (at most BAND_T) from the state s0: the totals
-// composed pairwise (thread t ends a run of 2 * off of them), so that hundreds
-// of them cost eight rounds instead of a matrix-vector product each in a row
-// (488 of them: 20 us).
-template <typename VT, int W>
-__device__ __forceinline__ void band_apply_pairwise(const VT *agg, int cnt, VT *sm, VT *s_state, VT (&s0)[W]) {
-    constexpr int E = W * W + W;
-    const int tid = threadIdx.x;
-    VT Mt[W][W], ct[W];
-#pragma unroll
-    for (int r = 0; r < W; ++r) {
-#pragma unroll
-        for (int q = 0; q < W; ++q) Mt[r][q] = r == q ? VT(1) : VT(0);
-        ct[r] = 0;
-    }
-    if (tid < cnt) {
-        const VT *t = agg + (long long)tid * E;
-#pragma unroll
-        for (int r = 0; r < W; ++r) {
-#pragma unroll
-            for (int q = 0; q < W; ++q) Mt[r][q] = __ldcg(t + r * W + q);
-            ct[r] = __ldcg(t + W * W + r);
-        }
-    }
-    for (int off = 1; off < BAND_T; off <<= 1) {
-        if ((tid & (off - 1)) == off - 1) band_put<VT, W>(sm, BAND_T, tid, Mt, ct);
-        __syncthreads();
-        if ((tid & (2 * off - 1)) == 2 * off - 1) {
-            VT Me[W][W], ce[W], nM[W][W], nc[W];
-            band_get<VT, W>(sm, BAND_T, tid - off, Me, ce);
-#pragma unroll
-            for (int r = 0; r < W; ++r) {
-                VT v = ct[r];
-#pragma unroll
-                for (int k = 0; k < W; ++k) v += Mt[r][k] * ce[k];
-                nc[r] = v;
-#pragma unroll
-                for (int q = 0; q < W; ++q) {
-                    VT u = 0;
-#pragma unroll
-                    for (int k = 0; k < W; ++k) u += Mt[r][k] * Me[k][q];
-                    nM[r][q] = u;
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < W; ++r) {
-                ct[r] = nc[r];
-#pragma unroll
-                for (int q = 0; q < W; ++q) Mt[r][q] = nM[r][q];
-            }
-        }
-        __syncthreads();
-    }
-    if (tid == BAND_T - 1) {
-#pragma unroll
-        for (int r = 0; r < W; ++r) {
-            VT v = ct[r];
-#pragma unroll
-            for (int k = 0; k < W; ++k) v += Mt[r][k] * s0[k];
-            s_state[r] = v;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < W; ++r) s0[r] = s_state[r];
-}
-
 // One launch per triangle (or per matrix).  Several right-hand sides run side
 // by side: column c = blockIdx.y, with its own CTA totals at agg + c * nblk *
 // (W*W+W) and its own ticket and ready flags (flags: c * (nblk + 1), the
 // ticket first, then one flag per CTA; zeroed before the launch).  Row p of
 // column c is element p * rs + c * cs of b and x: a work vector's, or the
 // caller's own (BT = double, rs = 1 or -1) where the rows are solved in the
-// caller's order or its reverse.  bounded: the totals of several CTAs may be
-// composed with one another.  Waits are bounded: after
-// `limit` polls a CTA raises RBS_STATUS_TIMEOUT and goes on.
-template <typename VT, int W, typename BT>
+// caller's order or its reverse.  BOUNDED: the totals of several CTAs may be
+// composed with one another (up to W = 4: wider maps do not fit the registers;
+// a template argument, as a branch at run time cost W = 1 up to 9 %: 33.9 -> 37.1
+// us for 6,000 rows in FP32).  Waits end: after `limit` polls a CTA raises
+// RBS_STATUS_TIMEOUT and goes on.
+template <typename VT, int W, typename BT, bool BOUNDED>
 __global__ void __launch_bounds__(BAND_T) k_band_onepass(const VT *__restrict__ coef, const VT *__restrict__ inv,
                                                          const BT *__restrict__ b, long long rs, long long cs, int m,
                                                          int C, int nch, VT *__restrict__ agg, int *flags, BT *x,
-                                                         int *status, long long limit, int bounded) {
+                                                         int *status, long long limit) {
     extern __shared__ unsigned char smem_raw[];
     VT *sm = reinterpret_cast<VT *>(smem_raw);
     __shared__ VT s_state[W];
@@ -289,8 +224,67 @@ __global__ void __launch_bounds__(BAND_T) k_band_onepass(const VT *__restrict__ 
                 if (it > 16) __nanosleep(64);
             }
         }
-        if (W <= 4 && bounded) {  // wider maps do not fit the registers
-            if constexpr (W <= 4) band_apply_pairwise<VT, W>(agg + (long long)base * E, cnt, sm, s_state, s0);
+        if constexpr (BOUNDED) {
+            // the totals composed pairwise (thread t ends a run of 2 * off of
+            // them), so that hundreds of them cost eight rounds instead of a
+            // matrix-vector product each in a row (488 of them: 20 us)
+            VT Mt[W][W], ct[W];
+#pragma unroll
+            for (int r = 0; r < W; ++r) {
+#pragma unroll
+                for (int q = 0; q < W; ++q) Mt[r][q] = r == q ? VT(1) : VT(0);
+                ct[r] = 0;
+            }
+            if (tid < cnt) {
+                const VT *t = agg + (long long)(base + tid) * E;
+#pragma unroll
+                for (int r = 0; r < W; ++r) {
+#pragma unroll
+                    for (int q = 0; q < W; ++q) Mt[r][q] = __ldcg(t + r * W + q);
+                    ct[r] = __ldcg(t + W * W + r);
+                }
+            }
+            for (int off = 1; off < BAND_T; off <<= 1) {
+                if ((tid & (off - 1)) == off - 1) band_put<VT, W>(sm, BAND_T, tid, Mt, ct);
+                __syncthreads();
+                if ((tid & (2 * off - 1)) == 2 * off - 1) {
+                    VT Me[W][W], ce[W], nM[W][W], nc[W];
+                    band_get<VT, W>(sm, BAND_T, tid - off, Me, ce);
+#pragma unroll
+                    for (int r = 0; r < W; ++r) {
+                        VT v = ct[r];
+#pragma unroll
+                        for (int k = 0; k < W; ++k) v += Mt[r][k] * ce[k];
+                        nc[r] = v;
+#pragma unroll
+                        for (int q = 0; q < W; ++q) {
+                            VT u = 0;
+#pragma unroll
+                            for (int k = 0; k < W; ++k) u += Mt[r][k] * Me[k][q];
+                            nM[r][q] = u;
+                        }
+                    }
+#pragma unroll
+                    for (int r = 0; r < W; ++r) {
+                        ct[r] = nc[r];
+#pragma unroll
+                        for (int q = 0; q < W; ++q) Mt[r][q] = nM[r][q];
+                    }
+                }
+                __syncthreads();
+            }
+            if (tid == BAND_T - 1) {
+#pragma unroll
+                for (int r = 0; r < W; ++r) {
+                    VT v = ct[r];
+#pragma unroll
+                    for (int k = 0; k < W; ++k) v += Mt[r][k] * s0[k];
+                    s_state[r] = v;
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < W; ++r) s0[r] = s_state[r];
         } else {
             __syncthreads();
             for (int i = tid; i < cnt * E; i += BAND_T) sm[i] = __ldcg(agg + (long long)base * E + i);

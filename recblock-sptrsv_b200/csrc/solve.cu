@@ -777,8 +777,8 @@ bool band_maps_bounded(const double *coef, const double *inv, const ExecBlock &B
 
 // Band-scan triangle, or the whole matrix (see band.cuh): one launch over all
 // K right-hand sides; row p of column c at p * rs + c * cs of bb and xx.
-template <typename VT, int W, typename BT>
-int run_band(Plan &P, const ExecBlock &B, const BT *bb, BT *xx, long long rs, long long cs, int K, std::string &err) {
+template <typename VT, int W, typename BT, bool BOUNDED>
+int run_band_w(Plan &P, const ExecBlock &B, const BT *bb, BT *xx, long long rs, long long cs, int K, std::string &err) {
     DeviceState &D = *P.dev;
     cudaStream_t st = D.stream;
     const VT *coef = Pools<VT>::bcoef(D) + B.band_off;
@@ -789,7 +789,7 @@ int run_band(Plan &P, const ExecBlock &B, const BT *bb, BT *xx, long long rs, lo
     const size_t smem = (size_t)BAND_T * E * sizeof(VT);
     static std::atomic<unsigned long long> attr_set{0};
     if (!attr_done(attr_set)) {
-        CK(cudaFuncSetAttribute(k_band_onepass<VT, W, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(cudaFuncSetAttribute(k_band_onepass<VT, W, BT, BOUNDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_mark(attr_set);
     }
     const int nch = B.band_nch, nblk = band_blocks(nch);
@@ -797,10 +797,16 @@ int run_band(Plan &P, const ExecBlock &B, const BT *bb, BT *xx, long long rs, lo
     // and the CTAs' ready flags (nblk + 1 ints) in the states scratch
     int *flags = reinterpret_cast<int *>(states);
     CK(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)K * (nblk + 1), st));
-    k_band_onepass<VT, W, BT><<<dim3(nblk, K), BAND_T, smem, st>>>(coef, binv, bb, rs, cs, B.m, B.band_c, nch, maps, flags,
-                                                                xx, D.status, P.opt.spin_limit,
-                                                                D.band || D.band_bounded[(size_t)B.index]);
+    k_band_onepass<VT, W, BT, BOUNDED><<<dim3(nblk, K), BAND_T, smem, st>>>(coef, binv, bb, rs, cs, B.m, B.band_c, nch, maps,
+                                                                         flags, xx, D.status, P.opt.spin_limit);
     return RBS_OK;
+}
+
+template <typename VT, int W, typename BT>
+int run_band(Plan &P, const ExecBlock &B, const BT *bb, BT *xx, long long rs, long long cs, int K, std::string &err) {
+    if constexpr (W <= 4)
+        if (P.dev->band || P.dev->band_bounded[(size_t)B.index]) return run_band_w<VT, W, BT, true>(P, B, bb, xx, rs, cs, K, err);
+    return run_band_w<VT, W, BT, false>(P, B, bb, xx, rs, cs, K, err);
 }
 
 template <typename VT, typename BT>
